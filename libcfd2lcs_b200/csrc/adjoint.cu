@@ -1508,10 +1508,13 @@ class Adjoint {
         SplineAxis<T> &D = sa_.ax[a];
         D.n = A.n;
         D.k = A.k;
-        const std::vector<lcsdata_t> pull = spline_pull_table(A);
+        const std::vector<lcsdata_t> pull = spline_pull_table(A), pullT = spline_pull_table_transposed(pull, A.n);
+        spline_fit_shape<T>(pull, A.n, A.k, false, FITB_MAX_WARM, D);
         if (!(D.t = upload(A.t, msg)) || !(D.rinv = upload(A.rinv, msg)) || !(D.tu = upload(A.tu, msg)) || !(D.pull = upload(pull, msg)))
           return false;
-        if (!(ptr_[a] = upload(spline_pull_table_transposed(pull, A.n), msg))) return false;
+        axT_[a] = D;
+        spline_fit_shape<T>(pullT, A.n, A.k, true, FITB_MAX_WARM, axT_[a]);
+        if (!(axT_[a].pull = upload(pullT, msg))) return false;
       }
     }
     ACK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
@@ -2051,11 +2054,11 @@ class Adjoint {
   bool cubic_ = false;
   bool flags_ = false;  // boundary flags (walls, slip, inflow / outflow, masks, 2-D)
   SplineAxes<T> sa_{};
-  T *ptr_[3] = {nullptr, nullptr, nullptr};
   std::vector<T *> Cl_, Cb_, DC_;
   T *blend_[4][3] = {};
   T *cfm_[3] = {nullptr, nullptr, nullptr};
   T *dcfm_[3] = {nullptr, nullptr, nullptr};
+  SplineAxis<T> axT_[3]{};  // the axes with the transposed factors
 
   // coefficients of the padded fields src into dst (the library's fit: x, then y, then z)
   void fit3(T *const src[3], T *const dst[3]) {
@@ -2067,13 +2070,19 @@ class Adjoint {
       d.f[c] = dst[c];
     }
     const int sx = dg_.P.sx, sxy = dg_.P.sxy, ny = dg_.P.n[1] + 2, nz = dg_.P.n[2] + 2;
-    const long warps = (long)((ny + 31) / 32) * nz;
-    const size_t smem = sizeof(T) * 4 * 2 * 32 * (XFIT_W + 1);
-    k_fit_xlines<T, 4><<<dim3((unsigned)((warps + 3) / 4), 3), 128, smem, stream_>>>(sa_.ax[0], s, d, ny, nz, (long)sx, (long)sxy);
-    k_fit_lines<T, 4><<<dim3((unsigned)(((long)sx * nz + 255) / 256), 3), 256, 0, stream_>>>(sa_.ax[1], di, d, sx, (long)sx * nz,
-                                                                                             (long)sx, (long)sxy);
-    k_fit_lines<T, 4><<<dim3((unsigned)(((long)sxy + 255) / 256), 3), 256, 0, stream_>>>(sa_.ax[2], di, d, sxy, (long)sxy, (long)sxy,
-                                                                                         (long)sxy);
+    for (int ax = 0; ax < 3; ax++) {
+      const SplineAxis<T> &A = sa_.ax[ax];
+      const FieldPtrs<T> &in = ax == 0 ? s : di;
+      if (fit_block<T, 4, false>(A, in, d, ax, sx, sxy, ny, nz, stream_)) continue;
+      if (ax == 0) {
+        const long warps = (long)((ny + 31) / 32) * nz;
+        const size_t smem = sizeof(T) * 4 * 2 * 32 * (XFIT_W + 1);
+        k_fit_xlines<T, 4><<<dim3((unsigned)((warps + 3) / 4), 3), 128, smem, stream_>>>(A, in, d, ny, nz, (long)sx, (long)sxy);
+      } else {
+        const long nfast = ax == 1 ? sx : sxy, nlines = ax == 1 ? (long)sx * nz : (long)sxy;
+        k_fit_lines<T, 4><<<dim3((unsigned)((nlines + 255) / 256), 3), 256, 0, stream_>>>(A, in, d, (int)nfast, nlines, nfast, (long)sxy);
+      }
+    }
   }
 
   // adjoint of fit3, in place: the transposed passes z, then y, then x
@@ -2082,11 +2091,16 @@ class Adjoint {
     for (int c = 0; c < 3; c++) d.f[c] = f[c];
     const long sx = dg_.P.sx, sxy = dg_.P.sxy;
     const int ny = dg_.P.n[1] + 2, nz = dg_.P.n[2] + 2;
-    k_fit_transpose<T><<<dim3((unsigned)((sxy + 255) / 256), 3), 256, 0, stream_>>>(ptr_[2], sa_.ax[2].n, d, (int)sxy, sxy, 1L, sxy, sxy);
-    k_fit_transpose<T><<<dim3((unsigned)((sx * nz + 255) / 256), 3), 256, 0, stream_>>>(ptr_[1], sa_.ax[1].n, d, (int)sx, sx * nz, 1L, sxy,
-                                                                                        sx);
-    k_fit_transpose<T><<<dim3((unsigned)(((long)ny * nz + 255) / 256), 3), 256, 0, stream_>>>(ptr_[0], sa_.ax[0].n, d, ny, (long)ny * nz,
-                                                                                              sx, sxy, 1L);
+    FieldPtrs<T> in{};
+    for (int c = 0; c < 3; c++) in.f[c] = f[c];
+    for (int ax = 2; ax >= 0; ax--) {
+      const SplineAxis<T> &A = axT_[ax];
+      if (fit_block<T, 4, true>(A, in, d, ax, sx, sxy, ny, nz, stream_)) continue;
+      const long nlines = ax == 0 ? (long)ny * nz : (ax == 1 ? sx * nz : sxy);
+      const int nfast = ax == 0 ? ny : (int)(ax == 1 ? sx : sxy);
+      k_fit_transpose<T><<<dim3((unsigned)((nlines + 255) / 256), 3), 256, 0, stream_>>>(A.pull, A.n, d, nfast, nlines, ax == 0 ? sx : 1L, sxy,
+                                                                                          ax == 0 ? 1L : (ax == 1 ? sx : sxy));
+    }
   }
 
   dim3 node_grid4() const { return dim3((dg_.P.n[0] + 31) / 32, (dg_.P.n[1] + 3) / 4, dg_.P.n[2]); }

@@ -1185,12 +1185,14 @@ class Engine : public EngineBase {
         return false;
       }
       SplineAxis<T> &D = s.axes.ax[a];
+      const std::vector<lcsdata_t> pull = pull_table(A);
       D.n = A.n;
       D.k = A.k;
+      spline_fit_shape<T>(pull, A.n, A.k, false, FITB_MAX_WARM, D);
       if (!(D.t = upload(A.t, msg))) return false;
       if (!(D.rinv = upload(A.rinv, msg))) return false;
       if (!(D.tu = upload(A.tu, msg))) return false;
-      if (!(D.pull = upload(pull_table(A), msg))) return false;
+      if (!(D.pull = upload(pull, msg))) return false;
     }
     L.sp[deg] = s;
     return true;
@@ -1210,17 +1212,19 @@ class Engine : public EngineBase {
         return false;
       }
       SplineAxis<T> &D = s.axes.ax[a];
+      const std::vector<lcsdata_t> pull = pull_table(A);
       D.n = A.n;
       D.k = A.k;
+      spline_fit_shape<T>(pull, A.n, A.k, false, FITB_MAX_WARM, D);
       if (!(D.t = upload(A.t, msg))) return false;
       if (!(D.rinv = upload(A.rinv, msg))) return false;
       if (!(D.tu = upload(A.tu, msg))) return false;
-      const std::vector<lcsdata_t> pull = pull_table(A);
       if (!(D.pull = upload(pull, msg))) return false;
       // the velocity fits solve with the LU factors rounded to the velocity type
       SplineAxis<TV> &E = sv.axes.ax[a];
       E.n = A.n;
       E.k = A.k;
+      spline_fit_shape<TV>(pull, A.n, A.k, false, FITB_MAX_WARM, E);
       if (!(E.t = upload<TV>(A.t, msg))) return false;
       if (!(E.rinv = upload<TV>(A.rinv, msg))) return false;
       if (!(E.tu = upload<TV>(A.tu, msg))) return false;
@@ -1236,6 +1240,10 @@ class Engine : public EngineBase {
   template <typename D, int K>
   void fit_pass(const SplineAxis<D> &A, FieldPtrs<D> s, FieldPtrsW<D> d, int axis, const DevGrid<T> &g) {
     const int sx = g.P.sx, sxy = g.P.sxy, ny = g.P.n[1] + 2, nz = g.P.n[2] + 2;
+    // an axis of three points (two-dimensional grids) has order 2, whose coefficients are the values
+    if (axis != 0 && A.identity) return;
+    counters_.kernel_launches++;
+    if (fit_block<D, K, false>(A, s, d, axis, sx, sxy, ny, nz, stream_)) return;
     if (axis == 0) {
       const long warps = (long)((ny + 31) / 32) * nz;
       const size_t smem = sizeof(D) * 4 * 2 * 32 * (XFIT_W + 1);  // two 32 x (XFIT_W + 1) tiles per warp
@@ -1273,7 +1281,6 @@ class Engine : public EngineBase {
       di.f[c] = dst[c];
       d.f[c] = dst[c];
     }
-    counters_.kernel_launches += 3;
     fit_pass_any(S.ax[0], s, d, 0, g);
     fit_pass_any(S.ax[1], di, d, 1, g);
     fit_pass_any(S.ax[2], di, d, 2, g);

@@ -1178,4 +1178,258 @@ __global__ void __launch_bounds__(128) k_fit_xlines(SplineAxis<T> A, const __gri
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// One axis' banded solves with each line cut into chunks that are swept at the same time, with
+// the bits of the whole-line sweeps.  The homogeneous part of either sweep decays along the line
+// (0.268 per element for the cubic on an even grid), so a sweep started from a zero window `warm`
+// elements before a chunk arrives there within rounding of the whole-line sweep, and nearly always
+// with its very bits (the host measures `warm` on the axis' own factors, spline_fit_warmup).
+// Nearly always is checked: the window a chunk started from must equal the values its neighbour
+// ended with, chunk by chunk from the line's end; a line that fails (a constant line can: two
+// neighbouring numbers may both be fixed points of the rounded recurrence) is swept again from the
+// right window.  A block stages LINES whole lines in shared memory and gives each of its 256 /
+// LINES chunks to LINES threads, thread = line:
+//   forward: warm-up over the source values before the chunk, barrier, the chunk in place;
+//   backward: warm-up over the forward values behind the chunk, barrier, the chunk in place.
+// Every element is read once and written once per axis, where the whole-line sweeps of
+// k_fit_lines / k_fit_xlines read and write it twice and run one dependent chain per line (a plane
+// of 1003 x 489 nodes has only 9000 lines to run side by side).
+// ADJ: the transposed solve (pivot in the forward sweep, spline_pull_table_transposed).
+// ---------------------------------------------------------------------------------------
+constexpr int FITB_THREADS = 256;
+
+// row pitch of the staged tile: x lines are copied along the row and swept across it
+template <bool XPASS, int LINES>
+__host__ __device__ constexpr int fitb_pitch() {
+  return XPASS ? LINES + 1 : LINES;
+}
+
+// One element: the sweeps of pull_forward / pull_backward, or the transposed ones (ADJ).  MID: a
+// row whose second and third off-diagonal factors are zero (every interior row: at its knot a
+// cubic's collocation row has three entries).
+template <typename T, int K, bool FWD, bool ADJ, bool MID>
+__device__ __forceinline__ T fit_step(const T *__restrict__ pc, int i0, T b, T (&win)[3]) {
+  if constexpr (MID) {
+    const T *c = pc + 8 * i0;
+    b = b - win[0] * __ldg(c + (FWD ? 0 : 3));
+    if (FWD == ADJ) b = b * __ldg(c + 6);
+    win[2] = win[1];
+    win[1] = win[0];
+    win[0] = b;
+    return b;
+  } else if constexpr (!ADJ) {
+    if constexpr (FWD) return pull_forward<T, K>(pc, i0, b, win);
+    else return pull_backward<T, K>(pc, i0, b, win);
+  } else {
+    const T *c = pc + 8 * i0 + (FWD ? 0 : 3);
+    b = b - win[0] * __ldg(c) - win[1] * __ldg(c + 1) - win[2] * __ldg(c + 2);
+    if (FWD) b = b * __ldg(pc + 8 * i0 + 6);
+    win[2] = win[1];
+    win[1] = win[0];
+    win[0] = b;
+    return b;
+  }
+}
+
+// the elements [a, b) of a staged column (from: the values read, to: where they are kept, when
+// STORE) in sweep order
+template <typename T, int K, bool FWD, bool ADJ, bool MID, bool STORE>
+__device__ __forceinline__ void fit_run(const T *__restrict__ pc, const T *from, long fp, T *to, int tp, int a, int b, T (&win)[3]) {
+  constexpr int G = 4;
+  const int step = FWD ? 1 : -1;
+  int e = FWD ? a : b - 1;
+  int left = b - a;
+  for (; left >= G; left -= G, e += G * step) {
+    T v[G];
+#pragma unroll
+    for (int q = 0; q < G; q++) v[q] = from[(e + q * step) * fp];
+#pragma unroll
+    for (int q = 0; q < G; q++) v[q] = fit_step<T, K, FWD, ADJ, MID>(pc, e + q * step, v[q], win);
+    if (STORE) {
+#pragma unroll
+      for (int q = 0; q < G; q++) to[(e + q * step) * tp] = v[q];
+    }
+  }
+  for (; left > 0; left--, e += step) {
+    const T v = fit_step<T, K, FWD, ADJ, MID>(pc, e, from[e * fp], win);
+    if (STORE) to[e * tp] = v;
+  }
+}
+
+// [a, b) split into the rows before, in and after [m0, m1), the rows with one off-diagonal factor
+template <typename T, int K, bool FWD, bool ADJ, bool STORE>
+__device__ __forceinline__ void fit_sweep(const T *__restrict__ pc, const T *from, long fp, T *to, int tp, int a, int b, int m0, int m1,
+                                          T (&win)[3]) {
+  const int p = min(max(m0, a), b), q = min(max(m1, p), b);
+  if (FWD) {
+    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, a, p, win);
+    fit_run<T, K, FWD, ADJ, true, STORE>(pc, from, fp, to, tp, p, q, win);
+    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, q, b, win);
+  } else {
+    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, q, b, win);
+    fit_run<T, K, FWD, ADJ, true, STORE>(pc, from, fp, to, tp, p, q, win);
+    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, a, p, win);
+  }
+}
+
+// bitwise comparison (a NaN equals itself)
+__device__ __forceinline__ bool same_bits(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_int(a) == __float_as_int(b); }
+
+// XPASS: line L is the contiguous row at L * es.  Else line L starts at L % nfast + (L / nfast) *
+// so and its elements are es apart.
+template <typename T, int K, bool XPASS, bool ADJ, int LINES>
+__global__ void __launch_bounds__(FITB_THREADS, 3)
+    k_fit_block(const T *__restrict__ pc, int n, int warm, int m0, int m1, const __grid_constant__ FieldPtrs<T> src,
+                const __grid_constant__ FieldPtrsW<T> dst, long nfast, long nlines, long es, long so) {
+  extern __shared__ __align__(16) unsigned char fit_smem[];
+  T *const tile = reinterpret_cast<T *>(fit_smem);
+  constexpr int P = fitb_pitch<XPASS, LINES>(), NCH = FITB_THREADS / LINES;
+  const int ln = threadIdx.x % LINES, ck = threadIdx.x / LINES;
+  const long L0 = (long)blockIdx.x * LINES;
+  const int nl = (int)min((long)LINES, nlines - L0);
+  const T *const s = src.f[blockIdx.y];
+  T *const d = dst.f[blockIdx.y];
+  // threads past the last line repeat it and write nothing
+  const long L = L0 + min(ln, nl - 1);
+  const long off = XPASS ? L * es : L % nfast + (L / nfast) * so;
+  const long ep = XPASS ? 1 : es;
+  if (XPASS) {
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < LINES; r += FITB_THREADS / 32) {
+      const T *row = s + (L0 + min(r, nl - 1)) * es;
+      for (int e = lane; e < n; e += 32) cp_async_elem(tile + e * P + r, row + e);
+    }
+  } else {
+    const T *p = s + off;
+    for (int e = ck; e < n; e += NCH) cp_async_elem(tile + e * P + ln, p + (long)e * es);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int ch = (n + NCH - 1) / NCH;
+  const int c0 = min(ck * ch, n), c1 = min(c0 + ch, n);
+  const bool some = c0 < c1;
+  T *const col = tile + ln;
+  T wf[3] = {T(0), T(0), T(0)}, win[3];
+  // --- forward ---
+  if (some) fit_sweep<T, K, true, ADJ, false>(pc, col, P, col, P, max(c0 - warm, 0), c0, m0, m1, wf);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 3; q++) win[q] = wf[q];
+  fit_sweep<T, K, true, ADJ, true>(pc, col, P, col, P, c0, c1, m0, m1, win);
+  __syncthreads();
+  // the window this chunk has to start from: the last values of the chunk before it
+  auto before = [&](T (&w)[3]) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) w[q] = q < K - 1 && c0 - 1 - q >= 0 ? col[(c0 - 1 - q) * P] : T(0);
+  };
+  auto behind = [&](T (&w)[3]) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) w[q] = q < K - 1 && c1 + q < n ? col[(c1 + q) * P] : T(0);
+  };
+  auto differs = [&](const T (&a)[3], const T (&b)[3]) {
+    bool r = false;
+#pragma unroll
+    for (int q = 0; q < K - 1; q++) r = r || !same_bits(a[q], b[q]);
+    return r;
+  };
+  before(win);
+  if (__syncthreads_or(some && c0 > 0 && differs(win, wf))) {
+    for (int c = 1; c < NCH; c++) {
+      if (ck == c && some) {
+        before(win);
+        if (differs(win, wf)) {
+#pragma unroll
+          for (int q = 0; q < 3; q++) wf[q] = win[q];
+          fit_sweep<T, K, true, ADJ, true>(pc, s + off, ep, col, P, c0, c1, m0, m1, win);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // --- backward ---
+  T wb[3] = {T(0), T(0), T(0)};
+  if (some) fit_sweep<T, K, false, ADJ, false>(pc, col, P, col, P, c1, min(c1 + warm, n), m0, m1, wb);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 3; q++) win[q] = wb[q];
+  fit_sweep<T, K, false, ADJ, true>(pc, col, P, col, P, c0, c1, m0, m1, win);
+  __syncthreads();
+  behind(win);
+  if (__syncthreads_or(some && c1 < n && differs(win, wb))) {
+    for (int c = NCH - 2; c >= 0; c--) {
+      if (ck == c && some) {
+        behind(win);
+        if (differs(win, wb)) {
+          // the chunk's forward values again (the source is still whole), then backward
+          fit_sweep<T, K, true, ADJ, true>(pc, s + off, ep, col, P, c0, c1, m0, m1, wf);
+          fit_sweep<T, K, false, ADJ, true>(pc, col, P, col, P, c0, c1, m0, m1, win);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (XPASS) {
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < nl; r += FITB_THREADS / 32) {
+      T *row = d + (L0 + r) * es;
+      for (int e = lane; e < n; e += 32) row[e] = tile[e * P + r];
+    }
+  } else if (ln < nl) {
+    T *p = d + off;
+    for (int e = ck; e < n; e += NCH) p[(long)e * es] = tile[e * P + ln];
+  }
+}
+
+// Lines per block of k_fit_block on an axis of n elements: 32 while two blocks fit an SM, then 16
+// and 8; 0 where the whole-line sweeps run: longer lines, factors that decay too slowly for the
+// warm-up to pay (strongly graded grids), and the y and z passes of k_fit_lines' own range.  Those
+// passes are coalesced as they are; they lose where there are too few lines to fill the GPU, or
+// where a field is larger than L2 so that their second sweep reads it from HBM again.  Measured on
+// B200 (FP64, three components, us, whole-line sweep against this):
+//   x: 48^3 22.8 / 10.5, 101x75x50 39 / 15, 173x160x147 137 / 81, 256^3 511 / 274, 1001x487x8 456 / 134
+//   y: 48^3 14.6 / 10.5, 101x75x50 18.7 / 20.5, 128^3 42 / 46, 200^3 190 / 135, 256^3 342 / 305,
+//      1001x487x8 151 / 93;  z of 8 planes (1001x487x8): 74 / 381
+// Bound by the L1/shared data pipe on large grids (65 to 76 % at 256^3, DRAM 34 %: the staged
+// values of a chunk are read for its neighbours' warm-ups too).
+constexpr int FITB_MAX_WARM = 96;
+template <typename T>
+inline int fit_block_lines(int n, int warm, int axis, long nlines) {
+  if (warm <= 0 || warm > FITB_MAX_WARM) return 0;
+  if (axis != 0 && (n < 24 || (nlines > 5000 && 3.0 * n * nlines * sizeof(T) < 128e6))) return 0;
+  for (int lines = 32; lines >= 8; lines /= 2)
+    if ((size_t)n * (lines + 1) * sizeof(T) <= 112 * 1024) return lines;
+  return 0;
+}
+
+template <typename T, int K, bool ADJ, int LINES>
+inline void fit_block_launch(const SplineAxis<T> &A, const FieldPtrs<T> &s, const FieldPtrsW<T> &d, int axis, long sx, long sxy, long ny,
+                             long nz, cudaStream_t stream) {
+  const long nlines = axis == 0 ? ny * nz : (axis == 1 ? sx * nz : sxy);
+  const dim3 grd((unsigned)((nlines + LINES - 1) / LINES), 3);
+  const size_t smem = (size_t)A.n * (axis == 0 ? LINES + 1 : LINES) * sizeof(T);
+  if (axis == 0) {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_fit_block<T, K, true, ADJ, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_fit_block<T, K, true, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, nlines, nlines, sx, 0);
+  } else {
+    const long es = axis == 1 ? sx : sxy;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_fit_block<T, K, false, ADJ, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_fit_block<T, K, false, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, es, nlines, es, sxy);
+  }
+}
+
+// one axis of a 3-component padded field (in place where s and d are the same); false where
+// k_fit_block does not apply
+template <typename T, int K, bool ADJ>
+inline bool fit_block(const SplineAxis<T> &A, const FieldPtrs<T> &s, const FieldPtrsW<T> &d, int axis, long sx, long sxy, long ny, long nz,
+                      cudaStream_t stream) {
+  switch (fit_block_lines<T>(A.n, A.warm, axis, axis == 0 ? ny * nz : (axis == 1 ? sx * nz : sxy))) {
+    case 32: fit_block_launch<T, K, ADJ, 32>(A, s, d, axis, sx, sxy, ny, nz, stream); return true;
+    case 16: fit_block_launch<T, K, ADJ, 16>(A, s, d, axis, sx, sxy, ny, nz, stream); return true;
+    case 8: fit_block_launch<T, K, ADJ, 8>(A, s, d, axis, sx, sxy, ny, nz, stream); return true;
+  }
+  return false;
+}
+
 }  // namespace cfd2lcs

@@ -24,6 +24,9 @@ template <typename T>
 struct SplineAxis {
   int n;          // points along the axis (interior + 2 ghosts)
   int k;          // order (degree + 1)
+  // of the fit's factors (spline_fit_shape): elements after which either sweep has forgotten its
+  // start, the rows [mid0, mid1) with one off-diagonal factor, and whether the fit changes nothing
+  int warm, mid0, mid1, identity;
   const T *t;     // n + k knots
   const T *rinv;  // per interval l (1-based, stored at l-1): 1/(t(l+r) - t(l+r-j)), 6 slots
   const T *pull;  // band LU of the collocation matrix in pull form, 8 values per element

@@ -1,6 +1,8 @@
 // Host set-up of a B-spline interpolation axis (knots, band LU, reciprocal spans).
 #pragma once
 
+#include <algorithm>
+#include <cmath>
 #include <vector>
 
 namespace cfd2lcs {
@@ -50,6 +52,63 @@ std::vector<R> spline_pull_table_transposed(const std::vector<R> &p, int n) {
     t[(size_t)8 * r + 6] = p[(size_t)8 * r + 6];
   }
   return t;
+}
+
+// Elements after which both sweeps of a pull table (either form) have forgotten the window they
+// started from: the smallest w such that, from every element of the line, a unit value in any
+// entry of the window before it has fallen below tol, in every entry, w elements further on.
+// 0 where some start needs more than `most`.  The device starts the sweeps of a line's chunks w
+// elements early from a zero window (k_fit_block).
+template <typename R>
+int spline_fit_warmup(const std::vector<R> &p, int n, int k, bool transposed, double tol, int most) {
+  int worst = 1;
+  for (int dir = 0; dir < 2; dir++)
+    for (int s = 0; s < n; s++)
+      for (int b = 0; b < k - 1; b++) {
+        double w[3] = {0, 0, 0};
+        w[b] = 1;
+        int m = 0;
+        while (true) {
+          double top = 0;
+          for (int j = 0; j < k - 1; j++) top = std::max(top, std::fabs(w[j]));
+          if (top <= tol || s + m >= n) break;
+          if (m >= most) return 0;
+          const int r = dir == 0 ? s + m : n - 1 - (s + m);
+          const R *c = &p[(size_t)8 * r];
+          double v = 0;
+          for (int j = 0; j < k - 1; j++) v -= w[j] * (double)c[(dir == 0 ? 0 : 3) + j];
+          if ((dir == 1) != transposed) v *= (double)c[6];
+          w[2] = w[1];
+          w[1] = w[0];
+          w[0] = v;
+          m++;
+        }
+        worst = std::max(worst, m);
+      }
+  return worst;
+}
+
+// What k_fit_block reads of an axis' factors, for a fit in type D (Axis: warm, mid0, mid1, identity).
+// The warm-up reaches 20 (FP64) or 11 (FP32) binary places below the last one: once the sweeps from
+// the zero window and from the whole line differ by less than a last place, each further element
+// rounds them to the same value with probability above one half.  Shorter warm-ups repeat more
+// lines, longer ones cost every chunk: at 2^-53 alone one chunk in 400 differed, here none of 10^5.
+template <typename D, typename R, typename Axis>
+void spline_fit_shape(const std::vector<R> &p, int n, int k, bool transposed, int most, Axis &A) {
+  A.warm = spline_fit_warmup(p, n, k, transposed, sizeof(D) == 8 ? 0x1p-73 : 0x1p-35, most);
+  auto wide = [&](int r) { return p[(size_t)8 * r + 1] != R(0) || p[(size_t)8 * r + 2] != R(0) || p[(size_t)8 * r + 4] != R(0) || p[(size_t)8 * r + 5] != R(0); };
+  // the longest run of rows with one factor on either side (the ends of a not-a-knot line have more)
+  A.mid0 = A.mid1 = 0;
+  for (int r = 0, run = 0; r < n; r++) {
+    run = wide(r) ? 0 : run + 1;
+    if (run > A.mid1 - A.mid0) A.mid0 = r + 1 - run, A.mid1 = r + 1;
+  }
+  A.identity = 1;
+  for (int r = 0; r < n; r++) {
+    for (int j = 0; j < 6; j++)
+      if (p[(size_t)8 * r + j] != R(0)) A.identity = 0;
+    if (p[(size_t)8 * r + 6] != R(1)) A.identity = 0;
+  }
 }
 
 }  // namespace cfd2lcs
