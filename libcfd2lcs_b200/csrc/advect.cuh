@@ -328,7 +328,7 @@ __device__ __forceinline__ void sample_velocity(const DevGrid<T> &g, const Splin
       out[c] = tse_ls_apply<T, INTERP == INTERP_CTSE_LIMIT>(g, x, no, [&](int p) { return T(omc * __ldg(a + p) + ct * __ldg(b + p)); });
     }
   } else {
-    constexpr int KC = INTERP == INTERP_SPLINE4 ? 4 : 0;
+    constexpr int KC = spline_orders(INTERP);
     SplineStencil<T> st;
     if (!spline_stencil<T, KC, UNI>(g, sa, x, no, st)) {
       out[0] = out[1] = out[2] = T(0);
@@ -378,7 +378,7 @@ __device__ __forceinline__ void sample_field(const DevGrid<T> &g, const SplineAx
       out[c] = tse_ls_apply<T, INTERP == INTERP_CTSE_LIMIT>(g, x, no, [&](int p) { return __ldg(fc + p); });
     }
   } else {
-    constexpr int KC = INTERP == INTERP_SPLINE4 ? 4 : 0;
+    constexpr int KC = spline_orders(INTERP);
     SplineStencil<T> st;
     if (!spline_stencil<T, KC, UNI>(g, sa, x, no, st)) {
       out[0] = out[1] = out[2] = T(0);

@@ -20,6 +20,7 @@ enum : int {
 
 enum { EULER_ = 0, TRAPEZOIDAL_ = 1, RK2_ = 2, RK3_ = 3, RK4_ = 4 };
 // INTERP_SPLINE: B-spline of any order per axis; INTERP_SPLINE4: cubic on every axis (3-D grid);
+// INTERP_SPLINE442: cubic in x and y, order 2 in z (two-dimensional grid, z singleton);
 // INTERP_TSE / INTERP_TSE_LIMIT: Taylor series about the tracked node, without / with limiter;
 // INTERP_CTSE / INTERP_CTSE_LIMIT: the same on a non-rectilinear grid (least-squares gradients,
 // full coordinate arrays), the only interpolators the reference runs there
@@ -31,10 +32,16 @@ enum {
   INTERP_TSE = 4,
   INTERP_TSE_LIMIT = 5,
   INTERP_CTSE = 6,
-  INTERP_CTSE_LIMIT = 7
+  INTERP_CTSE_LIMIT = 7,
+  INTERP_SPLINE442 = 8
 };
 
-__host__ __device__ constexpr bool interp_is_spline(int interp) { return interp == INTERP_SPLINE || interp == INTERP_SPLINE4; }
+__host__ __device__ constexpr bool interp_is_spline(int interp) {
+  return interp == INTERP_SPLINE || interp == INTERP_SPLINE4 || interp == INTERP_SPLINE442;
+}
+// the spline orders a B-spline variant fixes at compile time (spline.cuh): 4 on every axis, 4, 4 and
+// 2, or 0 (read from the axes)
+__host__ __device__ constexpr int spline_orders(int interp) { return interp == INTERP_SPLINE4 ? 4 : (interp == INTERP_SPLINE442 ? 442 : 0); }
 __host__ __device__ constexpr bool interp_is_curv(int interp) { return interp == INTERP_CTSE || interp == INTERP_CTSE_LIMIT; }
 
 template <typename T>

@@ -1240,8 +1240,6 @@ class Engine : public EngineBase {
   template <typename D, int K>
   void fit_pass(const SplineAxis<D> &A, FieldPtrs<D> s, FieldPtrsW<D> d, int axis, const DevGrid<T> &g) {
     const int sx = g.P.sx, sxy = g.P.sxy, ny = g.P.n[1] + 2, nz = g.P.n[2] + 2;
-    // an axis of three points (two-dimensional grids) has order 2, whose coefficients are the values
-    if (axis != 0 && A.identity) return;
     counters_.kernel_launches++;
     if (fit_block<D, K, false>(A, s, d, axis, sx, sxy, ny, nz, stream_)) return;
     if (axis == 0) {
@@ -1302,6 +1300,8 @@ class Engine : public EngineBase {
     if (interp == TSE) return INTERP_TSE;
     if (interp == TSE_LIMIT) return INTERP_TSE_LIMIT;
     if (sa.ax[0].k == 4 && sa.ax[1].k == 4 && sa.ax[2].k == 4) return INTERP_SPLINE4;
+    // a plane in x and y (its singleton z ghosts carry flags)
+    if (sa.ax[0].k == 4 && sa.ax[1].k == 4 && sa.ax[2].k == 2 && dg_.P.has_flags) return INTERP_SPLINE442;
     return INTERP_SPLINE;
   }
 
@@ -1874,6 +1874,7 @@ class Engine : public EngineBase {
     else if (iv == INTERP_CTSE) F ? sl_integ<INTERP_CTSE, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_CTSE, false>(sa, V, fo, fn, S, dt);
     else if (iv == INTERP_CTSE_LIMIT)
       F ? sl_integ<INTERP_CTSE_LIMIT, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_CTSE_LIMIT, false>(sa, V, fo, fn, S, dt);
+    else if (iv == INTERP_SPLINE442) sl_integ<INTERP_SPLINE442, true>(sa, V, fo, fn, S, dt);
     else if (iv == INTERP_SPLINE4) F ? sl_integ<INTERP_SPLINE4, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_SPLINE4, false>(sa, V, fo, fn, S, dt);
     else F ? sl_integ<INTERP_SPLINE, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_SPLINE, false>(sa, V, fo, fn, S, dt);
     CK(cudaGetLastError());
@@ -1906,6 +1907,7 @@ class Engine : public EngineBase {
     else if (iv == INTERP_CTSE) F ? fwd_integ<INTERP_CTSE, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_CTSE, false>(sa, V, P, S, dt, n);
     else if (iv == INTERP_CTSE_LIMIT)
       F ? fwd_integ<INTERP_CTSE_LIMIT, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_CTSE_LIMIT, false>(sa, V, P, S, dt, n);
+    else if (iv == INTERP_SPLINE442) fwd_integ<INTERP_SPLINE442, true>(sa, V, P, S, dt, n);
     else if (iv == INTERP_SPLINE4) F ? fwd_integ<INTERP_SPLINE4, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_SPLINE4, false>(sa, V, P, S, dt, n);
     else F ? fwd_integ<INTERP_SPLINE, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_SPLINE, false>(sa, V, P, S, dt, n);
     CK(cudaGetLastError());
@@ -2034,6 +2036,7 @@ class Engine : public EngineBase {
     else if (iv == INTERP_TSE_LIMIT) { if (F) COMPOSE(INTERP_TSE_LIMIT, true); else COMPOSE(INTERP_TSE_LIMIT, false); }
     else if (iv == INTERP_CTSE) { if (F) COMPOSE(INTERP_CTSE, true); else COMPOSE(INTERP_CTSE, false); }
     else if (iv == INTERP_CTSE_LIMIT) { if (F) COMPOSE(INTERP_CTSE_LIMIT, true); else COMPOSE(INTERP_CTSE_LIMIT, false); }
+    else if (iv == INTERP_SPLINE442 && F) COMPOSE(INTERP_SPLINE442, true);
     else if (iv == INTERP_SPLINE4) { if (F) COMPOSE(INTERP_SPLINE4, true); else COMPOSE(INTERP_SPLINE4, false); }
     else { if (F) COMPOSE(INTERP_SPLINE, true); else COMPOSE(INTERP_SPLINE, false); }
 #undef COMPOSE

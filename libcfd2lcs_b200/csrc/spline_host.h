@@ -88,7 +88,7 @@ int spline_fit_warmup(const std::vector<R> &p, int n, int k, bool transposed, do
   return worst;
 }
 
-// What k_fit_block reads of an axis' factors, for a fit in type D (Axis: warm, mid0, mid1, identity).
+// What k_fit_block reads of an axis' factors, for a fit in type D (Axis: warm, mid0, mid1).
 // The warm-up reaches 20 (FP64) or 11 (FP32) binary places below the last one: once the sweeps from
 // the zero window and from the whole line differ by less than a last place, each further element
 // rounds them to the same value with probability above one half.  Shorter warm-ups repeat more
@@ -102,12 +102,6 @@ void spline_fit_shape(const std::vector<R> &p, int n, int k, bool transposed, in
   for (int r = 0, run = 0; r < n; r++) {
     run = wide(r) ? 0 : run + 1;
     if (run > A.mid1 - A.mid0) A.mid0 = r + 1 - run, A.mid1 = r + 1;
-  }
-  A.identity = 1;
-  for (int r = 0; r < n; r++) {
-    for (int j = 0; j < 6; j++)
-      if (p[(size_t)8 * r + j] != R(0)) A.identity = 0;
-    if (p[(size_t)8 * r + 6] != R(1)) A.identity = 0;
   }
 }
 
