@@ -18,11 +18,11 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.environ.get("CFD2LCS_B200_BUILDDIR") or os.path.join(HERE, "_build")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["engine.cu", "engine_mixed.cu", "adjoint.cu", "grid.cpp", "spline_host.cpp", "writer.cpp", "capi.cpp"]
+SOURCES = ["engine.cu", "engine_mixed.cu", "backward.cu", "forward.cu", "refined.cu", "adjoint.cu", "grid.cpp", "spline_host.cpp", "writer.cpp", "capi.cpp"]
 # the FP64 FMA micro-benchmark bench.py reports the B-spline kernels against: a separate
 # measurement library, not part of the drop-in
 PROBE_SOURCE = "probe.cu"
-HEADERS = ["grid.h", "engine.h", "engine_impl.cuh", "adjoint.h", "device_common.cuh", "advect.cuh", "spline.cuh", "kernels.cuh", "tile.cuh", "eig3.h", "spline_host.h", "writer.h"]
+HEADERS = ["grid.h", "engine.h", "engine_impl.cuh", "launch.h", "adjoint.h", "device_common.cuh", "advect.cuh", "spline.cuh", "kernels.cuh", "tile.cuh", "eig3.h", "spline_host.h", "writer.h"]
 
 
 def lib_path(prec: str) -> str:

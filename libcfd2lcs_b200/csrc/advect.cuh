@@ -126,8 +126,22 @@ __device__ __forceinline__ int lin_corner(const LinStencil<T> &st, int c) {
   return st.p0 + ((c & 1) ? st.s[0] : 0) + ((c & 2) ? st.s[1] : 0) + ((c & 4) ? st.s[2] : 0);
 }
 
-template <typename T, typename V>
+// PLANE: on a grid whose z axis is a singleton a point stays on its plane (t = 1 exactly) unless the
+// caller's w moves it off, so the four lower corners have weight 0 and are left out there: half the
+// loads and sums, the same value.
+template <typename T, bool PLANE>
+__device__ __forceinline__ bool lin_flat(const LinStencil<T> &st) {
+  return PLANE && st.w[0] == T(0) && st.w[1] == T(0) && st.w[2] == T(0) && st.w[3] == T(0);
+}
+
+template <typename T, bool PLANE = false, typename V>
 __device__ __forceinline__ T lin_contract(const LinStencil<T> &st, V v) {
+  if (PLANE && lin_flat<T, PLANE>(st)) {  // (the chain below from its fifth term, one rounding each)
+    T acc = mul_rn(st.w[4], v(4));
+#pragma unroll
+    for (int c = 5; c < 8; c++) acc = fma_rn(st.w[c], v(c), acc);
+    return acc;
+  }
   return st.w[0] * v(0) + st.w[1] * v(1) + st.w[2] * v(2) + st.w[3] * v(3) + st.w[4] * v(4) + st.w[5] * v(5) + st.w[6] * v(6) +
          st.w[7] * v(7);
 }
@@ -140,9 +154,17 @@ __device__ __forceinline__ T lin_apply(const LinStencil<T> &st, const T *__restr
 // time-blended field u = (1-ct) u_n + ct u_np1 at the corners, then trilinear; TV is the
 // velocity storage type (FP32 in the mixed-precision form, weights rounded to it).  va(c), vb(c)
 // return corner c of u_n and u_np1.
-template <typename T, typename TV, typename VA, typename VB>
+template <typename T, typename TV, bool PLANE = false, typename VA, typename VB>
 __device__ __forceinline__ TV lin_blend_contract(const LinStencil<T> &st, TV omc, TV ct, VA va, VB vb) {
   TV acc = TV(0);
+  if (PLANE && lin_flat<T, PLANE>(st)) {
+#pragma unroll
+    for (int c = 4; c < 8; c++) {
+      const TV v = omc * va(c) + ct * vb(c);
+      acc = c == 4 ? mul_rn(TV(st.w[4]), v) : fma_rn(TV(st.w[c]), v, acc);
+    }
+    return acc;
+  }
 #pragma unroll
   for (int c = 0; c < 8; c++) {
     const TV v = omc * va(c) + ct * vb(c);
@@ -399,6 +421,13 @@ __device__ __forceinline__ void sample_field(const DevGrid<T> &g, const SplineAx
 // ---------------------------------------------------------------------------------------
 struct StageTimes {
   double ct[4];
+};
+
+// the stage fractions of the consecutive subcycles one launch advances (k_sl_run, k_fwd_run)
+constexpr int STAGE_RUN = 16;
+struct StageRun {
+  StageTimes s[STAGE_RUN];
+  int n;
 };
 
 // AT_NODE: xn is the coordinate of node no (first stage by sample_velocity_node)

@@ -18,6 +18,7 @@
 
 #include "grid.h"
 #include "kernels.cuh"
+#include "launch.h"
 #include "tile.cuh"
 #include "spline_host.h"
 #include "writer.h"
@@ -246,6 +247,7 @@ class Engine : public EngineBase {
     if (const char *e = std::getenv("CFD2LCS_B200_COMPOSE_MINB")) compose_minb_ = std::atoi(e) >= 4 ? 4 : 2;
     if (const char *e = std::getenv("CFD2LCS_B200_SL_TILE")) tile_mode_ = std::max(0, std::min(2, std::atoi(e)));
     if (const char *e = std::getenv("CFD2LCS_B200_SL_MARCH")) sl_march_ = std::atoi(e) != 0;
+    if (const char *e = std::getenv("CFD2LCS_B200_RUN")) run_ = std::atoi(e) != 0;
     if (const char *e = std::getenv("CFD2LCS_B200_SORT_EVERY")) sort_every_ = std::max(0, std::atoi(e));
     if (const char *e = std::getenv("CFD2LCS_B200_SL_MARCH_KC")) sl_march_kc_ = std::max(0, std::atoi(e));
     for (int a = 0; a < 3; a++) n_[a] = n[a];
@@ -279,6 +281,8 @@ class Engine : public EngineBase {
       }
     if (!(stage_ = arena_.alloc<lcsdata_t>((size_t)3 * N_, msg))) return false;
     if (!(red_ = arena_.alloc<DevReduce>(1, msg))) return false;
+    if (!(sl_run_bar_ = arena_.alloc<unsigned>(1, msg))) return false;
+    CK(cudaMemsetAsync(sl_run_bar_, 0, sizeof(unsigned), stream_));
     CK(cudaMemsetAsync(red_, 0, sizeof(DevReduce), stream_));
     CK(cudaStreamSynchronize(stream_));
     first_call_ = true;
@@ -575,11 +579,44 @@ class Engine : public EngineBase {
       if (!mark(adv0, msg)) return false;
       lcsdata_t lp_time = d.type == FTLE_BKWD ? t_np1_ : t_n_;
       const int kkind = d.type == FTLE_BKWD ? SPAN_SL : SPAN_FWD;
-      for (long sc = 0; sc < nsub; sc++) {
+      // sets whose stages need no field written between subcycles advance several per launch
+      const bool blended = spline || (interp == LINEAR && N_ >= lin_blend_min_ && (d.type != FTLE_BKWD || d.lg));
+      const bool run = d.type == FTLE_BKWD ? sl_run_usable(d, interp, V) : !blended;
+      for (long sc = 0; run && sc < nsub;) {
+        if (d.type == FTLE_FWD && sort_due(d, kRunSortInterval) && !timed_sort(d, msg)) return false;
+        StageRun R{};
+        const long left = d.type == FTLE_FWD ? std::max(1L, sort_room(d)) : (long)STAGE_RUN;
+        R.n = (int)std::min({nsub - sc, left, run_ ? (long)STAGE_RUN : 1L});
+        for (int q = 0; q < R.n; q++) {
+          R.s[q] = stage_times(lp_time, dt);
+          lp_time = lp_time + dt;
+          if (d.type == LP_TRACER) d.lifetime = d.lifetime + (lcsdata_t)std::fabs((double)dt);  // integrate_lp, lp_motion_m.f90:332
+        }
+        cudaEvent_t k0, k1;
+        if (!mark(k0, msg)) return false;
+        if (d.type == FTLE_BKWD) {
+          FieldPtrsW<T> fa, fb;
+          for (int c = 0; c < 3; c++) {
+            fa.f[c] = d.fm[d.cur][c];
+            fb.f[c] = d.fm[d.cur ^ 1][c];
+          }
+          CK((launch_sl_run<T, TV>(opt_->integrator, dg_.P.has_flags != 0, sl_run_block(), &sl_run_blocks_, stream_, dg_, V, fa, fb, R, (T)dt,
+                                   sl_run_bar_, &sl_run_arrivals_, &red_->err)));
+          d.cur ^= R.n & 1;
+          counters_.kernel_launches++;
+        } else if (!launch_fwd_run_set(iv, V, d, R, (T)dt, msg)) {
+          return false;
+        }
+        if (!mark(k1, msg)) return false;
+        const bool timed = d.type == FTLE_FWD;
+        spans_.push_back({k0, k1, kkind, -1, timed ? (int)(&d - diags_.data()) : -1, (int)std::min(d.since_sort, 1L << 30), R.n});
+        if (timed) d.since_sort += R.n;
+        sc += R.n;
+      }
+      for (long sc = 0; !run && sc < nsub; sc++) {
         cudaEvent_t k0, k1;
         StageTimes S = stage_times(lp_time, dt);
-        if ((spline || (interp == LINEAR && N_ >= lin_blend_min_ && (d.type != FTLE_BKWD || d.lg))) && !stage_blends(d, S, V, msg))
-          return false;
+        if (blended && !stage_blends(d, S, V, msg)) return false;
         if (d.type == FTLE_BKWD) {
           FieldPtrs<T> fo;
           FieldPtrsW<T> fn;
@@ -595,7 +632,7 @@ class Engine : public EngineBase {
             for (int c = 0; c < 3; c++) fo.f[c] = d.fmcoef[c];
           }
           if (!mark(k0, msg)) return false;
-          if (d.lg ? !launch_sl_refined(d, sa, spline ? d.lg->sp[deg].axes : SplineAxes<T>{}, V, fo, fn, S, (T)dt, msg)
+          if (d.lg ? !launch_sl_lcs(d, sa, spline ? d.lg->sp[deg].axes : SplineAxes<T>{}, V, fo, fn, S, (T)dt, msg)
                    : !launch_sl(iv, sa, V, fo, fn, S, (T)dt, msg))
             return false;
           if (!mark(k1, msg)) return false;
@@ -615,15 +652,13 @@ class Engine : public EngineBase {
           const bool resort = usable ? sc % sort_interval(interp) == 0 : sort_due(d);
           if (resort) {
             d.fwd_variant = usable ? tile_variant(1) : 0;
-            cudaEvent_t s0, s1;
-            if (!usable && !mark(s0, msg)) return false;
-            if (!sort_particles(d, msg, d.fwd_variant == 1)) return false;
             if (!usable) {
-              if (!mark(s1, msg)) return false;
-              spans_.push_back({s0, s1, SPAN_SORT, -1, di, 0});
+              if (!timed_sort(d, msg)) return false;
+            } else {
+              if (!sort_particles(d, msg, d.fwd_variant == 1)) return false;
+              d.since_sort = 0;
+              d.excess_ms = 0;
             }
-            d.since_sort = 0;
-            d.excess_ms = 0;
           }
           const bool staged = usable && d.fwd_variant == 1;
           if (!mark(k0, msg)) return false;
@@ -756,8 +791,9 @@ class Engine : public EngineBase {
         counters_.fwd_kernel_launches++;
         if (sp.diag >= 0 && sp.diag < (int)diags_.size()) {
           DiagT &d = diags_[sp.diag];
-          if (sp.since == 0 || d.base_ms < 0) d.base_ms = ms;
-          else d.excess_ms += std::max(0.0, (double)ms - d.base_ms);
+          const double each = (double)ms / sp.sub;  // per subcycle
+          if (sp.since == 0 || d.base_ms < 0) d.base_ms = each;
+          else d.excess_ms += sp.sub * std::max(0.0, each - d.base_ms);
         }
       } else if (sp.kind == SPAN_SORT) {
         if (sp.diag >= 0 && sp.diag < (int)diags_.size()) {
@@ -1050,6 +1086,7 @@ class Engine : public EngineBase {
     if (red_err_ & ERR_NONFINITE_VELOCITY) msg = "update: non-finite velocity (CFL number is not finite)";
     else if (red_err_ & ERR_TRACKING) msg = "ERROR: cannot locate all particles (node search did not converge)";
     else if (red_err_ & ERR_UNKNOWN_FLAG) msg = "ERROR: Unknown bcflag";
+    else if (red_err_ & ERR_GRID_BARRIER) msg = "device error: the blocks of a subcycle kernel did not meet";
     else if (red_err_ & ERR_ASYNC_COPY) msg = "device error: a shared-memory staging copy did not complete";
     else msg = "device error";
     return false;
@@ -1524,50 +1561,19 @@ class Engine : public EngineBase {
     return true;
   }
 
-  template <int INTERP, bool FS, bool FL>
-  void sl_refined_integ(DiagT &d, const SplineAxes<T> &sas, const SplineAxes<T> &sal, const VelFields<TV> &V, FieldPtrs<T> fo,
-                        FieldPtrsW<T> fn, StageTimes S, T dt) {
+  // sas: the solver grid's spline axes (velocity), sal: the lcs grid's (flow map); the kernel
+  // takes the all-cubic specialisation only when both grids allow it
+  bool launch_sl_lcs(DiagT &d, const SplineAxes<T> &sas, const SplineAxes<T> &sal, const VelFields<TV> &V, FieldPtrs<T> fo,
+                         FieldPtrsW<T> fn, StageTimes S, T dt, std::string &msg) {
+    const int interp = interpolator();
+    int iv = interp_variant(interp, sas);
+    if (interp_is_spline(iv)) iv = iv == INTERP_SPLINE4 && interp_variant(interp, sal) == INTERP_SPLINE4 ? INTERP_SPLINE4 : INTERP_SPLINE;
     LcsGrid<T> &L = *d.lg;
     FieldPtrs<T> pos{};
     for (int c = 0; c < 3; c++) pos.f[c] = L.pos[c];
-    const dim3 grd = node_grid(L.dg), blk(32, 8, 1);
-    int *err = &red_->err;
     counters_.kernel_launches++;
-#define SLR(IG)                                                                                                   \
-  k_sl_refined<T, TV, IG, INTERP, FS, FL><<<grd, blk, 0, stream_>>>(L.dg, dg_, sas, sal, pos, L.nos[0], L.nos[1], L.nos[2], V, fo, fn, \
-                                                                     S, dt, err)
-    switch (opt_->integrator) {
-      case 0: SLR(EULER_); break;
-      case 1: SLR(TRAPEZOIDAL_); break;
-      case 2: SLR(RK2_); break;
-      case 3: SLR(RK3_); break;
-      default: SLR(RK4_); break;
-    }
-#undef SLR
-  }
-
-  template <int INTERP>
-  void sl_refined_flags(DiagT &d, const SplineAxes<T> &sas, const SplineAxes<T> &sal, const VelFields<TV> &V, FieldPtrs<T> fo,
-                        FieldPtrsW<T> fn, StageTimes S, T dt) {
-    const bool FS = dg_.P.has_flags != 0, FL = d.lg->dg.P.has_flags != 0;
-    if (FS && FL) sl_refined_integ<INTERP, true, true>(d, sas, sal, V, fo, fn, S, dt);
-    else if (FS) sl_refined_integ<INTERP, true, false>(d, sas, sal, V, fo, fn, S, dt);
-    else if (FL) sl_refined_integ<INTERP, false, true>(d, sas, sal, V, fo, fn, S, dt);
-    else sl_refined_integ<INTERP, false, false>(d, sas, sal, V, fo, fn, S, dt);
-  }
-
-  // sas: the solver grid's spline axes (velocity), sal: the lcs grid's (flow map); the kernel
-  // takes the all-cubic specialisation only when both grids allow it
-  bool launch_sl_refined(DiagT &d, const SplineAxes<T> &sas, const SplineAxes<T> &sal, const VelFields<TV> &V, FieldPtrs<T> fo,
-                         FieldPtrsW<T> fn, StageTimes S, T dt, std::string &msg) {
-    const int interp = interpolator();
-    if (interp == NEAREST_NBR) sl_refined_flags<INTERP_NEAREST>(d, sas, sal, V, fo, fn, S, dt);
-    else if (interp == LINEAR) sl_refined_flags<INTERP_LINEAR>(d, sas, sal, V, fo, fn, S, dt);
-    else if (interp == TSE) sl_refined_flags<INTERP_TSE>(d, sas, sal, V, fo, fn, S, dt);
-    else if (interp == TSE_LIMIT) sl_refined_flags<INTERP_TSE_LIMIT>(d, sas, sal, V, fo, fn, S, dt);
-    else if (interp_variant(interp, sas) == INTERP_SPLINE4 && interp_variant(interp, sal) == INTERP_SPLINE4)
-      sl_refined_flags<INTERP_SPLINE4>(d, sas, sal, V, fo, fn, S, dt);
-    else sl_refined_flags<INTERP_SPLINE>(d, sas, sal, V, fo, fn, S, dt);
+    cfd2lcs::launch_sl_refined<T, TV>(iv, opt_->integrator, dg_.P.has_flags != 0, L.dg.P.has_flags != 0, node_grid(L.dg), dim3(32, 8, 1),
+                                      stream_, L.dg, dg_, sas, sal, pos, L.nos[0], L.nos[1], L.nos[2], V, fo, fn, S, dt, &red_->err);
     CK(cudaGetLastError());
     return true;
   }
@@ -1816,36 +1822,22 @@ class Engine : public EngineBase {
     return true;
   }
 
-  template <int INTERP, bool F>
-  void sl_integ(const SplineAxes<T> &sa, const VelFields<TV> &V, FieldPtrs<T> fo, FieldPtrsW<T> fn, StageTimes S, T dt) {
+  bool launch_sl(int iv, const SplineAxes<T> &sa, const VelFields<TV> &V, FieldPtrs<T> fo, FieldPtrsW<T> fn, StageTimes S, T dt,
+                 std::string &msg) {
+    const bool F = dg_.P.has_flags != 0;
     sl_variant_ = -1;
-    if constexpr (INTERP == INTERP_LINEAR) {
-      if (sl_tile_lin_usable(V, fo) && (sl_variant_ = tile_variant(0)) == 1) {
-        counters_.kernel_launches++;
-        counters_.sl_staged_launches++;
-        switch (opt_->integrator) {
-          case 0: launch_sl_tile_lin<EULER_, F>(V, fo, fn, S, dt); break;
-          case 1: launch_sl_tile_lin<TRAPEZOIDAL_, F>(V, fo, fn, S, dt); break;
-          case 2: launch_sl_tile_lin<RK2_, F>(V, fo, fn, S, dt); break;
-          case 3: launch_sl_tile_lin<RK3_, F>(V, fo, fn, S, dt); break;
-          default: launch_sl_tile_lin<RK4_, F>(V, fo, fn, S, dt); break;
-        }
-        return;
-      }
-    }
-    if constexpr (INTERP == INTERP_SPLINE4) {
-      if (sl_tile_usable(V, fo) && (sl_variant_ = tile_variant(0)) == 1) {
-        counters_.kernel_launches++;
-        counters_.sl_staged_launches++;
-        switch (opt_->integrator) {
-          case 0: launch_sl_tile<EULER_, F>(sa, V, fo, fn, S, dt); break;
-          case 1: launch_sl_tile<TRAPEZOIDAL_, F>(sa, V, fo, fn, S, dt); break;
-          case 2: launch_sl_tile<RK2_, F>(sa, V, fo, fn, S, dt); break;
-          case 3: launch_sl_tile<RK3_, F>(sa, V, fo, fn, S, dt); break;
-          default: launch_sl_tile<RK4_, F>(sa, V, fo, fn, S, dt); break;
-        }
-        return;
-      }
+    counters_.kernel_launches++;
+    const bool lin = iv == INTERP_LINEAR && sl_tile_lin_usable(V, fo), cub = iv == INTERP_SPLINE4 && sl_tile_usable(V, fo);
+    if ((lin || cub) && (sl_variant_ = tile_variant(0)) == 1) {
+      counters_.sl_staged_launches++;
+      for_flags(F, [&](auto FL) {
+        for_integrator(opt_->integrator, [&](auto IG) {
+          if (lin) launch_sl_tile_lin<decltype(IG)::value, decltype(FL)::value>(V, fo, fn, S, dt);
+          else launch_sl_tile<decltype(IG)::value, decltype(FL)::value>(sa, V, fo, fn, S, dt);
+        });
+      });
+      CK(cudaGetLastError());
+      return true;
     }
     // blocks of 32 x 8/bz x bz nodes: spanning z layers lets a block's warps share the corners
     // of the layers between them in L1.  Measured on B200 (bz = 1 / 2 / 4): FP64 velocity, ABC
@@ -1853,63 +1845,55 @@ class Engine : public EngineBase {
     // launch; FP32 velocity, ABC 256^3 2.81 / 2.79 / 2.96 ms.  Flat blocks on 2-D grids.
     const int bz = n_[2] < 8 ? 1 : (std::is_same<TV, float>::value ? 2 : 4), by = 8 / bz;
     const dim3 blk(32, by, bz), grd((n_[0] + 31) / 32, (n_[1] + by - 1) / by, (n_[2] + bz - 1) / bz);
-    int *err = &red_->err;
-    counters_.kernel_launches++;
-    switch (opt_->integrator) {
-      case 0: k_sl_subcycle<T, TV, EULER_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, fo, fn, S, dt, err); break;
-      case 1: k_sl_subcycle<T, TV, TRAPEZOIDAL_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, fo, fn, S, dt, err); break;
-      case 2: k_sl_subcycle<T, TV, RK2_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, fo, fn, S, dt, err); break;
-      case 3: k_sl_subcycle<T, TV, RK3_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, fo, fn, S, dt, err); break;
-      default: k_sl_subcycle<T, TV, RK4_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, fo, fn, S, dt, err); break;
-    }
-  }
-
-  bool launch_sl(int iv, const SplineAxes<T> &sa, const VelFields<TV> &V, FieldPtrs<T> fo, FieldPtrsW<T> fn, StageTimes S, T dt,
-                 std::string &msg) {
-    const bool F = dg_.P.has_flags != 0;
-    if (iv == INTERP_NEAREST) F ? sl_integ<INTERP_NEAREST, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_NEAREST, false>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_LINEAR) F ? sl_integ<INTERP_LINEAR, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_LINEAR, false>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_TSE) F ? sl_integ<INTERP_TSE, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_TSE, false>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_TSE_LIMIT) F ? sl_integ<INTERP_TSE_LIMIT, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_TSE_LIMIT, false>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_CTSE) F ? sl_integ<INTERP_CTSE, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_CTSE, false>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_CTSE_LIMIT)
-      F ? sl_integ<INTERP_CTSE_LIMIT, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_CTSE_LIMIT, false>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_SPLINE442) sl_integ<INTERP_SPLINE442, true>(sa, V, fo, fn, S, dt);
-    else if (iv == INTERP_SPLINE4) F ? sl_integ<INTERP_SPLINE4, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_SPLINE4, false>(sa, V, fo, fn, S, dt);
-    else F ? sl_integ<INTERP_SPLINE, true>(sa, V, fo, fn, S, dt) : sl_integ<INTERP_SPLINE, false>(sa, V, fo, fn, S, dt);
+    launch_sl_gather<T, TV>(iv, opt_->integrator, F, grd, blk, stream_, dg_, sa, V, fo, fn, S, dt, &red_->err);
     CK(cudaGetLastError());
     return true;
   }
 
-  template <int INTERP, bool F>
-  void fwd_integ(const SplineAxes<T> &sa, const VelFields<TV> &V, Particles<T> P, StageTimes S, T dt, int np) {
-    const int blk = 256, grd = (int)((np + blk - 1) / blk);
-    int *err = &red_->err;
-    counters_.kernel_launches++;
-    switch (opt_->integrator) {
-      case 0: k_fwd_subcycle<T, TV, EULER_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, P, S, dt, np, err); break;
-      case 1: k_fwd_subcycle<T, TV, TRAPEZOIDAL_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, P, S, dt, np, err); break;
-      case 2: k_fwd_subcycle<T, TV, RK2_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, P, S, dt, np, err); break;
-      case 3: k_fwd_subcycle<T, TV, RK3_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, P, S, dt, np, err); break;
-      default: k_fwd_subcycle<T, TV, RK4_, INTERP, F><<<grd, blk, 0, stream_>>>(dg_, sa, V, P, S, dt, np, err); break;
-    }
-  }
-
   bool launch_fwd(int iv, const SplineAxes<T> &sa, const VelFields<TV> &V, Particles<T> P, StageTimes S, T dt, std::string &msg,
                   long np = -1) {
-    const bool F = dg_.P.has_flags != 0;
     const int n = (int)(np < 0 ? N_ : np);
     if (n == 0) return true;
-    if (iv == INTERP_NEAREST) F ? fwd_integ<INTERP_NEAREST, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_NEAREST, false>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_LINEAR) F ? fwd_integ<INTERP_LINEAR, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_LINEAR, false>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_TSE) F ? fwd_integ<INTERP_TSE, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_TSE, false>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_TSE_LIMIT) F ? fwd_integ<INTERP_TSE_LIMIT, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_TSE_LIMIT, false>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_CTSE) F ? fwd_integ<INTERP_CTSE, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_CTSE, false>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_CTSE_LIMIT)
-      F ? fwd_integ<INTERP_CTSE_LIMIT, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_CTSE_LIMIT, false>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_SPLINE442) fwd_integ<INTERP_SPLINE442, true>(sa, V, P, S, dt, n);
-    else if (iv == INTERP_SPLINE4) F ? fwd_integ<INTERP_SPLINE4, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_SPLINE4, false>(sa, V, P, S, dt, n);
-    else F ? fwd_integ<INTERP_SPLINE, true>(sa, V, P, S, dt, n) : fwd_integ<INTERP_SPLINE, false>(sa, V, P, S, dt, n);
+    counters_.kernel_launches++;
+    launch_fwd_gather<T, TV>(iv, opt_->integrator, dg_.P.has_flags != 0, stream_, dg_, sa, V, P, S, dt, n, &red_->err);
+    CK(cudaGetLastError());
+    return true;
+  }
+
+  // Several subcycles per launch (k_sl_run, k_fwd_run); CFD2LCS_B200_RUN=0 at cfd2lcs_init advances
+  // one per launch.
+  bool run_ = true;
+  unsigned *sl_run_bar_ = nullptr, sl_run_arrivals_ = 0;
+  int sl_run_blocks_ = 0;  // blocks of k_sl_run resident at once (0: not asked yet)
+  int sl_run_opts_ = -1;   // the integrator that number belongs to
+
+  dim3 sl_run_block() const { return n_[2] < 8 ? dim3(32, 8, 1) : dim3(32, 2, 4); }
+
+  // Backward LINEAR sets on the solver grid of at most two tiles per resident block.  Not where the
+  // staged kernels are asked for (CFD2LCS_B200_SL_TILE=2).
+  bool sl_run_usable(const DiagT &d, int interp, const VelFields<TV> &V) {
+    if (!run_ || interp != LINEAR || d.lg || tile_mode_ == 2 || dg_.P.curv) return false;
+    const dim3 b = sl_run_block();
+    const long tiles = (long)((n_[0] + b.x - 1) / b.x) * ((n_[1] + b.y - 1) / b.y) * ((n_[2] + b.z - 1) / b.z);
+    // with other instances' kernels on the device, blocks that must all be resident at once wait for
+    // room: the batched form takes this kernel only where half the SMs hold them (the 16-instance
+    // batch took 23 ms per pass with every grid of up to 8 blocks per SM on it, 16.1 like this)
+    if (tiles > (opt_->shared_device ? num_sms_ / 2 : 4L * num_sms_)) return false;
+    if (sl_run_opts_ != opt_->integrator) {
+      sl_run_blocks_ = 0;
+      if (launch_sl_run<T, TV>(opt_->integrator, dg_.P.has_flags != 0, b, &sl_run_blocks_, stream_, dg_, V, {}, {}, {}, T(0), nullptr, nullptr,
+                               nullptr) != cudaSuccess)
+        sl_run_blocks_ = 0;
+      sl_run_opts_ = opt_->integrator;
+    }
+    return tiles <= 2L * sl_run_blocks_;
+  }
+
+  bool launch_fwd_run_set(int iv, const VelFields<TV> &V, const DiagT &d, const StageRun &R, T dt, std::string &msg) {
+    const int n = d.type == LP_TRACER ? d.np : (int)dN(d);
+    if (n == 0) return true;
+    counters_.kernel_launches++;
+    launch_fwd_run<T, TV>(iv, opt_->integrator, dg_.P.has_flags != 0, stream_, dg_, V, d.P, R, dt, n, &red_->err);
     CK(cudaGetLastError());
     return true;
   }
@@ -2318,10 +2302,28 @@ class Engine : public EngineBase {
   // instances keep the fixed interval: with other instances' kernels interleaved, a sort's event
   // span is not its cost (measured on the 64-instance batch: 89 ms per step with the rule, 81 ms
   // with the interval).
-  bool sort_due(const DiagT &d) const {
+  bool sort_due(const DiagT &d, long interval = kSortInterval) const {
     if (sort_every_ > 0) return d.since_sort >= sort_every_;
-    if (d.sort_ms <= 0 || opt_->shared_device) return d.since_sort >= kSortInterval;
+    if (d.sort_ms <= 0 || opt_->shared_device) return d.since_sort >= interval;
     return d.excess_ms >= d.sort_ms;
+  }
+  // The same for the sets that advance several subcycles per launch, whose interval before a sort has
+  // been timed (and in the batched form) is one full launch: their fields are small, and a sort is
+  // four launches.  Subcycles left until the next sort falls due:
+  static constexpr long kRunSortInterval = STAGE_RUN;
+  long sort_room(const DiagT &d) const {
+    if (sort_every_ > 0) return sort_every_ - d.since_sort;
+    if (d.sort_ms <= 0 || opt_->shared_device) return kRunSortInterval - d.since_sort;
+    return STAGE_RUN;
+  }
+  // a sort between event marks, for the sets on sort_due's schedule
+  bool timed_sort(DiagT &d, std::string &msg) {
+    cudaEvent_t s0, s1;
+    if (!mark(s0, msg) || !sort_particles(d, msg) || !mark(s1, msg)) return false;
+    spans_.push_back({s0, s1, SPAN_SORT, -1, (int)(&d - diags_.data()), 0});
+    d.since_sort = 0;
+    d.excess_ms = 0;
+    return true;
   }
   // fwd_tile: the 16 x 4 x 4-cell tiles the staged forward kernel reads, else the 32 x 4 x 2
   // tiles that suit the gathering kernel
@@ -2385,6 +2387,7 @@ class Engine : public EngineBase {
     int tune = -1;   // hot-kernel spans while the tuner samples: family * 2 + variant
     int diag = -1;   // forward launches and sorts of a set on the sort_due schedule: its index
     int since = 0;   // forward launches: subcycles since that set's last sort or reset
+    int sub = 1;     // subcycles the launch advanced
   };
   std::vector<cudaEvent_t> evpool_;
   size_t evnext_ = 0;

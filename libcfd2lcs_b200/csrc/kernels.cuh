@@ -336,14 +336,8 @@ __global__ void __launch_bounds__(256) k_reset_refined(DevGrid<T> gl, FieldPtrs<
 // periodic wrap of exchange_lpdata.  Thread q advances the particle in storage slot q.
 // ---------------------------------------------------------------------------------------
 template <typename T, typename TV, int INTEG, int INTERP, bool HAS_FLAGS>
-__global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_subcycle(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P, StageTimes S,
-                                                       T dt, int np, int *err) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= np) return;
-  T xn[3] = {P.x[0][q], P.x[1][q], P.x[2][q]};
-  int no[3] = {P.no[0][q], P.no[1][q], P.no[2][q]};
-  // the accumulated displacement is read up front, off the integration's dependent chain
-  const T dx0[3] = {P.dx[0][q], P.dx[1][q], P.dx[2][q]};
+__device__ __forceinline__ void fwd_advance(const DevGrid<T> &g, const SplineAxes<T> &sa, const VelFields<TV> &V, const StageTimes &S, T dt,
+                                            T xn[3], int no[3], T dx[3], int *err) {
   constexpr bool CURV = interp_is_curv(INTERP);
   T x[3];
   integrate<T, TV, INTEG, INTERP, false, particle_uniform_basis()>(g, sa, V, S, dt, xn, no, x);
@@ -355,11 +349,46 @@ __global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_subcycle(
     x[2] = xn[2];
   }
 #pragma unroll
-  for (int c = 0; c < 3; c++) P.dx[c][q] = dx0[c] + (x[c] - xn[c]);
+  for (int c = 0; c < 3; c++) dx[c] = dx[c] + (x[c] - xn[c]);
   track_pass<T, CURV>(g, x, no);
   wrap_particle(g, x, no);
 #pragma unroll
+  for (int c = 0; c < 3; c++) xn[c] = x[c];
+}
+
+template <typename T, typename TV, int INTEG, int INTERP, bool HAS_FLAGS>
+__global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_subcycle(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P, StageTimes S,
+                                                       T dt, int np, int *err) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= np) return;
+  T x[3] = {P.x[0][q], P.x[1][q], P.x[2][q]};
+  int no[3] = {P.no[0][q], P.no[1][q], P.no[2][q]};
+  // the accumulated displacement is read up front, off the integration's dependent chain
+  T dx[3] = {P.dx[0][q], P.dx[1][q], P.dx[2][q]};
+  fwd_advance<T, TV, INTEG, INTERP, HAS_FLAGS>(g, sa, V, S, dt, x, no, dx, err);
+#pragma unroll
   for (int c = 0; c < 3; c++) {
+    P.dx[c][q] = dx[c];
+    P.x[c][q] = x[c];
+    P.no[c][q] = no[c];
+  }
+}
+
+// The same for R.n consecutive subcycles, the particle in registers throughout: the sets whose
+// stages read the two velocity levels themselves (no blend fields to write between subcycles).
+// A particle depends on no other, so nothing has to meet between the subcycles.
+template <typename T, typename TV, int INTEG, int INTERP, bool HAS_FLAGS>
+__global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_run(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P,
+                                                  const __grid_constant__ StageRun R, T dt, int np, int *err) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= np) return;
+  T x[3] = {P.x[0][q], P.x[1][q], P.x[2][q]};
+  int no[3] = {P.no[0][q], P.no[1][q], P.no[2][q]};
+  T dx[3] = {P.dx[0][q], P.dx[1][q], P.dx[2][q]};
+  for (int s = 0; s < R.n; s++) fwd_advance<T, TV, INTEG, INTERP, HAS_FLAGS>(g, sa, V, R.s[s], dt, x, no, dx, err);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    P.dx[c][q] = dx[c];
     P.x[c][q] = x[c];
     P.no[c][q] = no[c];
   }

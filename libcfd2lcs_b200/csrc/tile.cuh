@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(SLT_THREADS, CFD2LCS_SLT_MINB)
 // component; u0 / u1 / fm (c, index) read component c of u_n, u_np1 and the flow map.  Every
 // staged LINEAR kernel runs this one expression, so they are bitwise equal to each other and to
 // k_sl_subcycle.
-template <typename T, typename TV, int INTEG, bool HAS_FLAGS, typename IV, typename IF, typename U0, typename U1, typename FM>
+template <typename T, typename TV, int INTEG, bool HAS_FLAGS, bool PLANE = false, typename IV, typename IF, typename U0, typename U1, typename FM>
 __device__ __forceinline__ void lin_sl_node(const DevGrid<T> &g, const StageTimes &S, T dt, int i, int j, int k, const T xn[3], const T lm[3],
                                             const T lc[3], const T lp[3], const T rm[3], const T rp[3], IV iv, IF ifm, U0 u0, U1 u1, FM fm,
                                             FieldPtrsW<T> fmn, int *err) {
@@ -495,7 +495,7 @@ __device__ __forceinline__ void lin_sl_node(const DevGrid<T> &g, const StageTime
       idx[c] = iv(st.i0[0] + ((c & 1) ? st.d[0] : 0), st.i0[1] + ((c & 2) ? st.d[1] : 0), st.i0[2] + ((c & 4) ? st.d[2] : 0));
 #pragma unroll
     for (int c = 0; c < 3; c++)
-      u[c] = T(lin_blend_contract<T, TV>(st, omc, ct, [&](int e) { return u0(c, idx[e]); }, [&](int e) { return u1(c, idx[e]); }));
+      u[c] = T(lin_blend_contract<T, TV, PLANE>(st, omc, ct, [&](int e) { return u0(c, idx[e]); }, [&](int e) { return u1(c, idx[e]); }));
   };
   T u[3], x[3];
   {  // first stage on the node (sample_velocity_node)
@@ -579,7 +579,7 @@ __device__ __forceinline__ void lin_sl_node(const DevGrid<T> &g, const StageTime
     idx[c] = ifm(st.i0[0] + ((c & 1) ? st.d[0] : 0), st.i0[1] + ((c & 2) ? st.d[1] : 0), st.i0[2] + ((c & 4) ? st.d[2] : 0));
   T fmp[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++) fmp[c] = lin_contract<T>(st, [&](int e) { return fm(c, idx[e]); });
+  for (int c = 0; c < 3; c++) fmp[c] = lin_contract<T, PLANE>(st, [&](int e) { return fm(c, idx[e]); });
   const int p = pidx(sx, sxy, i, j, k);
   const int fl = HAS_FLAGS ? (int)g.flag[p] : (int)LCS_INTERNAL;
   const T mask = fl != LCS_MASK ? T(1) : T(0);
@@ -592,6 +592,72 @@ __device__ __forceinline__ void lin_sl_node(const DevGrid<T> &g, const StageTime
     fmn.f[c][p] = vfin[c];
   }
   write_ghosts<T, HAS_FLAGS, GHOST_FM>(g, fmn.f, i, j, k, vpre, vfin, err);
+}
+
+// Arrival of every block of a cooperative launch at one barrier: *bar counts arrivals since the
+// buffer was cleared, target is the count at which the last block has come.  Gives up after about
+// one second of SM clock (2^31 cycles).
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target) {
+  __syncthreads();
+  bool ok = true;
+  if ((threadIdx.x | threadIdx.y | threadIdx.z) == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    const long long t0 = clock64();
+    unsigned v;
+    while (true) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if ((int)(v - target) >= 0) break;
+      if (clock64() - t0 > (1LL << 31)) {
+        ok = false;
+        break;
+      }
+    }
+  }
+  return __syncthreads_and(ok);
+}
+
+// K1 for R.n consecutive subcycles in one cooperative launch: LINEAR on grids of a few tiles per
+// SM.  There a subcycle is some microseconds of dependent operations, and its launch, its event
+// records and the refill of L1 and of the constant cache cost more than the work; here the velocity
+// levels and coordinate lines stay in L1 from one subcycle to the next and the blocks meet at a
+// barrier between them.  The flow maps fa and fb change roles every subcycle, so they are read
+// through L2 (ld.cg).  Measured on B200, double gyre 512 x 256 (RK2, FP64), per subcycle: 13.0 us
+// against 13.3 for the separate kernel and 30 with its launch and event records; 64 x 32: 7.5
+// against 10.7 and 60.  2 blocks of 256 per SM (no spills) and up to two tiles per block: 152 us per
+// 11.7 subcycles, 4 blocks and one tile 164.  The node routine
+// is the staged kernels' (lin_sl_node), so the bits are k_sl_subcycle's.  nt: tiles along each axis, dealt over the blocks.
+template <typename T, typename TV, int INTEG, bool HAS_FLAGS, bool PLANE>
+__global__ void __launch_bounds__(256, 2)
+    k_sl_run(DevGrid<T> g, VelFields<TV> V, FieldPtrsW<T> fa, FieldPtrsW<T> fb, const __grid_constant__ StageRun R, T dt, int3 nt, unsigned *bar,
+             unsigned base, int *err) {
+  for (int s = 0; s < R.n; s++) {
+    const FieldPtrsW<T> &src = (s & 1) ? fb : fa, &dst = (s & 1) ? fa : fb;
+    for (int t = blockIdx.x; t < nt.x * nt.y * nt.z; t += gridDim.x) {
+      const int i = (t % nt.x) * blockDim.x + threadIdx.x + 1, j = ((t / nt.x) % nt.y) * blockDim.y + threadIdx.y + 1,
+                k = (t / (nt.x * nt.y)) * blockDim.z + threadIdx.z + 1;
+      if (i > g.P.n[0] || j > g.P.n[1] || k > g.P.n[2]) continue;
+      const int nd[3] = {i, j, k};
+      T xn[3], lm[3], lc[3], lp[3], rm[3], rp[3];
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        xn[a] = __ldg(g.lt[a] + nd[a]);
+        lm[a] = __ldg(g.li[a] + nd[a] - 1);
+        lc[a] = __ldg(g.li[a] + nd[a]);
+        lp[a] = __ldg(g.li[a] + nd[a] + 1);
+        rm[a] = __ldg(g.ri[a] + nd[a] - 1);
+        rp[a] = __ldg(g.ri[a] + nd[a]);
+      }
+      auto at = [&](int x, int y, int z) { return pidx(g.P.sx, g.P.sxy, x, y, z); };
+      lin_sl_node<T, TV, INTEG, HAS_FLAGS, PLANE>(
+          g, R.s[s], dt, i, j, k, xn, lm, lc, lp, rm, rp, at, at, [&](int c, int e) { return __ldg(V.un[c] + e); },
+          [&](int c, int e) { return __ldg(V.unp1[c] + e); }, [&](int c, int e) { return __ldcg(src.f[c] + e); }, dst, err);
+    }
+    if (s + 1 < R.n && !grid_barrier(bar, base + (unsigned)(s + 1) * gridDim.x)) {
+      if ((threadIdx.x | threadIdx.y | threadIdx.z) == 0) atomicOr(err, ERR_GRID_BARRIER);
+      return;
+    }
+  }
 }
 
 using LinGeom = TileGeom<32, 4, 4, 1>;
