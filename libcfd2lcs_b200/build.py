@@ -22,7 +22,7 @@ SOURCES = ["engine.cu", "engine_mixed.cu", "backward.cu", "forward.cu", "refined
 # the FP64 FMA micro-benchmark bench.py reports the B-spline kernels against: a separate
 # measurement library, not part of the drop-in
 PROBE_SOURCE = "probe.cu"
-HEADERS = ["grid.h", "engine.h", "engine_impl.cuh", "launch.h", "adjoint.h", "device_common.cuh", "advect.cuh", "spline.cuh", "kernels.cuh", "tile.cuh", "eig3.h", "spline_host.h", "writer.h"]
+HEADERS = ["grid.h", "engine.h", "engine_impl.cuh", "launch.h", "scalar_ops.h", "adjoint.h", "device_common.cuh", "advect.cuh", "spline.cuh", "kernels.cuh", "tile.cuh", "eig3.h", "spline_host.h", "writer.h"]
 
 
 def lib_path(prec: str) -> str:

@@ -650,6 +650,26 @@ __device__ __forceinline__ bool track_pass_lines(const DevGrid<T> &g, const T x[
   // candidate's squared distance is then a sum of three register values; the 27 candidates
   // are unrolled with constant offsets.
   const int sa = g.P.single_axis;
+  bool inner = true;  // every line the scan looks at is an interior one
+#pragma unroll
+  for (int a = 0; a < 3; a++) inner = inner && (a == sa || (no[a] > 1 && no[a] < g.P.n[a]));
+  if (inner) {
+    T q[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+      for (int o = -1; o <= 1; o++) {
+        const T d = __ldg(g.lt[a] + no[a] + o) - x[a];
+        q[a][o + 1] = mul_rn(d, d);
+      }
+    int off[3];
+    if (nbr_scan_short(q, sa, off)) {
+      no[0] += off[0];
+      no[1] += off[1];
+      no[2] += off[2];
+      return off[0] != 0 || off[1] != 0 || off[2] != 0;
+    }
+  }
   T sqp[3][3], sqn[3][3];
   unsigned ok = 0;  // bit 3a+o+1: line no[a]+o is interior, or axis a is periodic
 #pragma unroll

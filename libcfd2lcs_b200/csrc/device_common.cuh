@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "grid.h"
+#include "scalar_ops.h"
 
 namespace cfd2lcs {
 
@@ -88,11 +89,9 @@ struct Particles {
 
 __device__ __forceinline__ int pidx(const int sx, const int sxy, int i, int j, int k) { return i + sx * j + sxy * k; }
 
-template <typename T>
-__device__ __forceinline__ T clamp01(T v) {
-  // max(min(v,1),0) of the reference; a NaN argument yields the bound as gfortran does
-  return fmax(fmin(v, T(1)), T(0));
-}
+// max(min(v,1),0) of the reference; a NaN argument yields the bound as gfortran does
+__device__ __forceinline__ double clamp01(double v) { return clamp01_select(v); }
+__device__ __forceinline__ float clamp01(float v) { return fmaxf(fminf(v, 1.0f), 0.0f); }
 
 // ---------------------------------------------------------------------------------------
 // Ghost fill of a padded field, written by the interior node that is the source of each
