@@ -1762,39 +1762,47 @@ class Engine : public EngineBase {
     return true;
   }
 
-  // The staged LINEAR backward kernel: k_sl_march_lin (planes marching along z) where every
-  // field has a tensor map and the velocity is stored in the flow map's type, else the boxes of
-  // k_sl_tile_lin.  CFD2LCS_B200_SL_MARCH=0 at cfd2lcs_init keeps the boxes;
+  // The staged LINEAR backward kernel: k_sl_march_lin (planes marching along z), its planes copied
+  // by TMA where every field has a tensor map, else element by element.  CFD2LCS_B200_SL_MARCH=0 at
+  // cfd2lcs_init takes the boxes of k_sl_tile_lin;
   // CFD2LCS_B200_SL_MARCH_KC sets the planes per column run (default: runs of 8..64 planes
   // giving about eight waves of two blocks per SM).
   bool sl_march_ = true;
   int sl_march_kc_ = 0;
   int num_sms_ = 148;
 
+  template <int IG, bool F, bool TMA>
+  void march_lin(const VelFields<TV> &V, FieldPtrs<T> fo, FieldPtrsW<T> fn, StageTimes S, T dt, const TileMaps &tm) {
+    auto *kernel = k_sl_march_lin<T, TV, IG, F, TMA>;
+    const size_t smem = slm_bytes<T, TV>() + 128;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const long cols = (long)((n_[0] + SLM_X - 1) / SLM_X) * ((n_[1] + SLM_Y - 1) / SLM_Y);
+    int kc = sl_march_kc_;
+    if (kc <= 0) kc = (int)std::max(8L, std::min(64L, (long)n_[2] * cols / (8L * 2 * num_sms_)));
+    kc = std::min(kc, n_[2]);
+    const dim3 blk(SLM_X, SLM_Y, 1), grd((n_[0] + SLM_X - 1) / SLM_X, (n_[1] + SLM_Y - 1) / SLM_Y, (n_[2] + kc - 1) / kc);
+    kernel<<<grd, blk, smem, stream_>>>(dg_, V, fo, fn, S, dt, kc, &red_->err, tm);
+    counters_.sl_march_launches++;
+  }
+
   template <int IG, bool F>
   bool launch_sl_march_lin(const VelFields<TV> &V, FieldPtrs<T> fo, FieldPtrsW<T> fn, StageTimes S, T dt) {
-    if constexpr (!std::is_same<T, TV>::value) {
-      return false;
-    } else {
-      // a box row (SLM_SX elements) must be a multiple of 16 bytes: FP64 only
-      if (!sl_march_ || (SLM_SX * sizeof(T)) % 16) return false;
-      TileMaps tm{};
-      for (int c = 0; c < 3; c++)
-        if (!tensor_map<T>(V.un[c], SLM_SX, SLM_SY, 1, tm.m[c]) || !tensor_map<T>(V.unp1[c], SLM_SX, SLM_SY, 1, tm.m[3 + c]) ||
-            !tensor_map<T>(fo.f[c], SLM_SX, SLM_SY, 1, tm.m[6 + c]))
-          return false;
-      tm.on = 1;
-      const long cols = (long)((n_[0] + SLM_X - 1) / SLM_X) * ((n_[1] + SLM_Y - 1) / SLM_Y);
-      int kc = sl_march_kc_;
-      if (kc <= 0) kc = (int)std::max(8L, std::min(64L, (long)n_[2] * cols / (8L * 2 * num_sms_)));
-      kc = std::min(kc, n_[2]);
-      const size_t smem = slm_bytes<T>() + 128;
-      cudaFuncSetAttribute(k_sl_march_lin<T, IG, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      const dim3 blk(SLM_X, SLM_Y, 1), grd((n_[0] + SLM_X - 1) / SLM_X, (n_[1] + SLM_Y - 1) / SLM_Y, (n_[2] + kc - 1) / kc);
-      k_sl_march_lin<T, IG, F><<<grd, blk, smem, stream_>>>(dg_, fn, S, dt, kc, &red_->err, tm);
-      counters_.sl_march_launches++;
-      return true;
+    if (!sl_march_) return false;
+    TileMaps tm{};
+    // a box row (SLM_SX elements) must be a multiple of 16 bytes: FP64 only
+    if constexpr (std::is_same<T, TV>::value && (SLM_SX * sizeof(T)) % 16 == 0) {
+      bool maps = true;
+      for (int c = 0; c < 3 && maps; c++)
+        maps = tensor_map<T>(V.un[c], SLM_SX, SLM_SY, 1, tm.m[c]) && tensor_map<T>(V.unp1[c], SLM_SX, SLM_SY, 1, tm.m[3 + c]) &&
+               tensor_map<T>(fo.f[c], SLM_SX, SLM_SY, 1, tm.m[6 + c]);
+      if (maps) {
+        tm.on = 1;
+        march_lin<IG, F, true>(V, fo, fn, S, dt, tm);
+        return true;
+      }
     }
+    march_lin<IG, F, false>(V, fo, fn, S, dt, tm);
+    return true;
   }
 
   template <int IG, bool F>

@@ -743,15 +743,23 @@ __global__ void __launch_bounds__(SLT_THREADS, CFD2LCS_SLL_MINB)
 }
 
 // ---------------------------------------------------------------------------------------
-// LINEAR backward subcycle marching along z (FP64 with tensor maps).  A block owns a column of
+// LINEAR backward subcycle marching along z.  A block owns a column of
 // 32 x 8 nodes over a run of kc planes and keeps a ring of four staged planes of all nine
 // components (u_n, u_np1, flow map; each plane 34 x 10 with its 1-node halo): while it works on
 // plane k from planes k-1, k and k+1, the copy of plane k+2 lands in the slot plane k-2 left.
 // Against the 32 x 4 x 4 boxes of k_sl_tile_lin (34 x 6 x 6 staged per 512 nodes, 2.4 staged
 // elements per node) a plane is staged once per column run, 1.33 elements per node in x and y,
 // plus two planes per run in z, and the block never waits for its copies but at the start of a
-// run.  Every copy lands on the mbarrier of its slot (one phase per plane that passes through
-// it); every wait is bounded.
+// run.  Two ways of copying a plane, chosen by the engine:
+//   TMA (FP64 with tensor maps, i.e. rows of a multiple of 16 bytes): one box copy per component
+//   and plane by thread 0, landing on the mbarrier of its slot (one phase per plane that passes
+//   through it); every wait is bounded;
+//   element copies (cp.async by all threads, 18 a thread and plane) for every other row length and
+//   for FP32 velocity or flow maps, whose boxes would otherwise be gathered or copied row by row.
+// Measured on B200, per launch, element copies against what these grids ran before: channel 191 x
+// 129 x 95 RK4 FP64 208 us against 212 (row-copied boxes); 200^3 RK2 in the single library 226
+// against 324 (gathering).  The FP64 form at 256^3 takes 444 us: 78 shared-memory reads of 8 bytes
+// per node are 288 us of that pipe.
 // ---------------------------------------------------------------------------------------
 constexpr int SLM_X = 32, SLM_Y = 8, SLM_SX = SLM_X + 2, SLM_SY = SLM_Y + 2, SLM_SLOTS = 4;
 constexpr int SLM_THREADS = SLM_X * SLM_Y;
@@ -760,42 +768,82 @@ template <typename T>
 __host__ __device__ constexpr int slm_comp() {
   return ((SLM_SX * SLM_SY * (int)sizeof(T) + 127) / 128) * 128 / (int)sizeof(T);
 }
-template <typename T>
+// shared memory of the ring: six velocity components and the flow map's three per slot
+template <typename T, typename TV>
 __host__ __device__ constexpr size_t slm_bytes() {
-  return (size_t)SLM_SLOTS * 9 * slm_comp<T>() * sizeof(T);
+  return (size_t)SLM_SLOTS * (6 * slm_comp<TV>() * sizeof(TV) + 3 * slm_comp<T>() * sizeof(T));
 }
 
+// resident blocks asked of the compiler: 2 (16 warps, 128 registers) in FP64, 3 in FP32 (2 / 3 / 4:
+// 243 / 226 / 252 us on the 200^3 case)
 #ifndef CFD2LCS_SLM_MINB
 #define CFD2LCS_SLM_MINB 2
 #endif
+#ifndef CFD2LCS_SLM_MINB_SP
+#define CFD2LCS_SLM_MINB_SP 3
+#endif
 
-template <typename T, int INTEG, bool HAS_FLAGS>
-__global__ void __launch_bounds__(SLM_THREADS, CFD2LCS_SLM_MINB)
-    k_sl_march_lin(DevGrid<T> g, FieldPtrsW<T> fmn, StageTimes S, T dt, int kc, int *err, const __grid_constant__ TileMaps tm) {
+template <typename T, typename TV, int INTEG, bool HAS_FLAGS, bool TMA>
+__global__ void __launch_bounds__(SLM_THREADS, sizeof(T) == 8 ? CFD2LCS_SLM_MINB : CFD2LCS_SLM_MINB_SP)
+    k_sl_march_lin(DevGrid<T> g, VelFields<TV> V, FieldPtrs<T> fmo, FieldPtrsW<T> fmn, StageTimes S, T dt, int kc, int *err,
+                   const __grid_constant__ TileMaps tm) {
   extern __shared__ __align__(128) unsigned char slm_smem_raw[];
-  T *const box = reinterpret_cast<T *>(smem_aligned128(slm_smem_raw));
+  constexpr int CS = slm_comp<T>(), CV = slm_comp<TV>();
+  // per slot: six velocity planes; then, for all slots, the flow map's three
+  TV *const boxv = reinterpret_cast<TV *>(smem_aligned128(slm_smem_raw));
+  T *const boxf = reinterpret_cast<T *>(boxv + (size_t)SLM_SLOTS * 6 * CV);
   __shared__ __align__(8) uint64_t bar[SLM_SLOTS];
-  constexpr int CS = slm_comp<T>();
-  constexpr unsigned PLANE_BYTES = 9u * (unsigned)(SLM_SX * SLM_SY * sizeof(T));
+  constexpr unsigned PLANE_BYTES = (unsigned)(SLM_SX * SLM_SY * (6 * sizeof(TV) + 3 * sizeof(T)));
   const int tid = threadIdx.x + SLM_X * threadIdx.y;
   const int xs = (int)blockIdx.x * SLM_X, ys = (int)blockIdx.y * SLM_Y;  // padded origin of the staged planes
   const int K0 = 1 + (int)blockIdx.z * kc, K1 = min(K0 + kc - 1, g.P.n[2]);
   // plane p (K0-1 <= p <= K1+1) sits in slot p & 3; its phase on that slot's barrier is the
   // parity of its pass through the ring
   auto parity = [&](int p) { return (unsigned)(((p - (K0 - 1)) >> 2) & 1); };
-  auto issue = [&](int p) {
-    T *const dst = box + (size_t)(p & 3) * 9 * CS;
-    mbar_arrive_expect_tx(&bar[p & 3], PLANE_BYTES);
+  // element copies: the staged elements tid and tid + 256 of a component plane, their offset in the
+  // padded plane (-1: outside the array, or past the staged plane)
+  int at[2] = {-1, -1};
+  if constexpr (!TMA) {
 #pragma unroll
-    for (int c = 0; c < 9; c++) tensor_copy_3d(dst + (size_t)c * CS, tm.m + c, xs, ys, p, &bar[p & 3]);
-  };
-  if (tid == 0) {
-#pragma unroll
-    for (int s = 0; s < SLM_SLOTS; s++) mbar_init(&bar[s], 1);
+    for (int m = 0; m < 2; m++) {
+      const int e = tid + m * SLM_THREADS, x = xs + e % SLM_SX, y = ys + e / SLM_SX;
+      if (e < SLM_SX * SLM_SY && x <= g.P.n[0] + 1 && y <= g.P.n[1] + 1) at[m] = x + y * g.P.sx;
+    }
   }
-  __syncthreads();
-  if (tid == 0)
-    for (int p = K0 - 1; p <= min(K0 + 1, K1 + 1); p++) issue(p);
+  auto issue = [&](int p) {
+    TV *const dv = boxv + (size_t)(p & 3) * 6 * CV;
+    T *const df = boxf + (size_t)(p & 3) * 3 * CS;
+    if constexpr (TMA) {
+      if (tid != 0) return;
+      mbar_arrive_expect_tx(&bar[p & 3], PLANE_BYTES);
+#pragma unroll
+      for (int c = 0; c < 6; c++) tensor_copy_3d(dv + (size_t)c * CV, tm.m + c, xs, ys, p, &bar[p & 3]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) tensor_copy_3d(df + (size_t)c * CS, tm.m + 6 + c, xs, ys, p, &bar[p & 3]);
+    } else {
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        if (at[m] < 0) continue;
+        const long q = at[m] + (long)p * g.P.sxy;
+        const int e = tid + m * SLM_THREADS;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          cp_async_elem(dv + c * CV + e, V.un[c] + q);
+          cp_async_elem(dv + (3 + c) * CV + e, V.unp1[c] + q);
+          cp_async_elem(df + c * CS + e, fmo.f[c] + q);
+        }
+      }
+      cp_async_commit();
+    }
+  };
+  if constexpr (TMA) {
+    if (tid == 0) {
+#pragma unroll
+      for (int s = 0; s < SLM_SLOTS; s++) mbar_init(&bar[s], 1);
+    }
+    __syncthreads();
+  }
+  for (int p = K0 - 1; p <= K0 + 1; p++) issue(p);  // (K1 + 1 >= K0 + 1)
 
   const int i = xs + 1 + (int)threadIdx.x, j = ys + 1 + (int)threadIdx.y;
   const bool ok = i <= g.P.n[0] && j <= g.P.n[1];
@@ -812,21 +860,26 @@ __global__ void __launch_bounds__(SLM_THREADS, CFD2LCS_SLM_MINB)
   rm[0] = __ldg(g.ri[0] + ni - 1), rp[0] = __ldg(g.ri[0] + ni);
   rm[1] = __ldg(g.ri[1] + nj - 1), rp[1] = __ldg(g.ri[1] + nj);
   T rz = __ldg(g.ri[2] + K0 - 1);
-  auto sidx = [&](int x, int y, int z) { return (z & 3) * 9 * CS + (y - ys) * SLM_SX + (x - xs); };
+  auto vidx = [&](int x, int y, int z) { return (z & 3) * 6 * CV + (y - ys) * SLM_SX + (x - xs); };
+  auto fidx = [&](int x, int y, int z) { return (z & 3) * 3 * CS + (y - ys) * SLM_SX + (x - xs); };
   for (int k = K0; k <= K1; k++) {
-    bool w = mbar_wait_bounded(&bar[(k + 1) & 3], parity(k + 1));
-    if (k == K0) w = mbar_wait_bounded(&bar[(k - 1) & 3], parity(k - 1)) && mbar_wait_bounded(&bar[k & 3], parity(k)) && w;
-    // the barrier also ends every thread's reads of plane k-2, whose slot the next copy fills
-    if (!__syncthreads_and(w)) {
-      if (tid == 0) atomicOr(err, ERR_ASYNC_COPY);
-      // let the copies in flight land before the block leaves
-      for (int p = max(K0 - 1, k - 1); p <= min(k + 1, K1 + 1); p++) mbar_wait_bounded(&bar[p & 3], parity(p));
-      return;
+    // planes k-1, k and k+1 have landed; the barrier also ends every thread's reads of plane k-2,
+    // whose slot the next copy fills
+    if constexpr (TMA) {
+      bool w = mbar_wait_bounded(&bar[(k + 1) & 3], parity(k + 1));
+      if (k == K0) w = mbar_wait_bounded(&bar[(k - 1) & 3], parity(k - 1)) && mbar_wait_bounded(&bar[k & 3], parity(k)) && w;
+      if (!__syncthreads_and(w)) {
+        if (tid == 0) atomicOr(err, ERR_ASYNC_COPY);
+        // let the copies in flight land before the block leaves
+        for (int p = max(K0 - 1, k - 1); p <= min(k + 1, K1 + 1); p++) mbar_wait_bounded(&bar[p & 3], parity(p));
+        return;
+      }
+      if (tid == 0 && k + 2 <= K1 + 1) fence_proxy_async_smem();
+    } else {
+      cp_async_wait<0>();  // at most plane k+1 is outstanding here
+      __syncthreads();
     }
-    if (tid == 0 && k + 2 <= K1 + 1) {
-      fence_proxy_async_smem();
-      issue(k + 2);
-    }
+    if (k + 2 <= K1 + 1) issue(k + 2);
     // z lines of this plane, rolled along the column
     lm[2] = zc;
     lc[2] = zp;
@@ -838,10 +891,9 @@ __global__ void __launch_bounds__(SLM_THREADS, CFD2LCS_SLM_MINB)
     rz = __ldg(g.ri[2] + k);
     rp[2] = rz;
     if (ok)
-      lin_sl_node<T, T, INTEG, HAS_FLAGS>(
-          g, S, dt, i, j, k, xn, lm, lc, lp, rm, rp, sidx, sidx, [&](int c, int e) { return box[(size_t)c * CS + e]; },
-          [&](int c, int e) { return box[(size_t)(3 + c) * CS + e]; }, [&](int c, int e) { return box[(size_t)(6 + c) * CS + e]; },
-          fmn, err);
+      lin_sl_node<T, TV, INTEG, HAS_FLAGS>(
+          g, S, dt, i, j, k, xn, lm, lc, lp, rm, rp, vidx, fidx, [&](int c, int e) { return boxv[c * CV + e]; },
+          [&](int c, int e) { return boxv[(3 + c) * CV + e]; }, [&](int c, int e) { return boxf[c * CS + e]; }, fmn, err);
   }
 }
 
