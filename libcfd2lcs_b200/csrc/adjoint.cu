@@ -24,6 +24,7 @@
 #include "adjoint.h"
 
 #include <algorithm>
+#include <mutex>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -49,26 +50,87 @@ namespace {
 enum { EULER = 0, TRAPEZOIDAL = 1, RK2 = 2, RK3 = 3, RK4 = 4 };
 enum { LINEAR_I = 1, CUBIC_I = 3 };
 
-// device memory of one adjoint call
+// Device memory of the adjoint calls.  cudaMalloc and cudaFree take 0.25 and 0.2 ms a buffer, and
+// milliseconds where hundreds of MB are mapped and unmapped: 18 of the 29 ms of a gradient at 80^3
+// (39 buffers, 0.4 GB).  The calls draw from one stream-ordered pool per device instead, which keeps up
+// to 1 GiB from one call to the next (an optimisation calls the gradient again and again); what is
+// above that goes back to the device when a call ends, the rest when the library is reset or finalised
+// (adjoint_release_memory).
+constexpr uint64_t POOL_KEEP = 1ull << 30;
+std::mutex g_pool_lock;
+cudaMemPool_t g_pools[64] = {};
+
+bool call_pool(cudaMemPool_t &pool, std::string &msg) {
+  int dev = 0;
+  ACK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) {
+    msg = "adjoint: device index out of range";
+    return false;
+  }
+  std::lock_guard<std::mutex> guard(g_pool_lock);
+  if (!g_pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    ACK(cudaMemPoolCreate(&p, &props));
+    uint64_t keep = POOL_KEEP;
+    ACK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+    g_pools[dev] = p;
+  }
+  pool = g_pools[dev];
+  return true;
+}
+
+// One call's buffers: taken and given back in the order of the call's stream, carved from chunks of
+// 32 MiB and more (larger requests alone).
 class Pool {
  public:
-  ~Pool() {
-    for (void *p : ptrs_) cudaFree(p);
+  bool open(cudaStream_t stream, std::string &msg) {
+    stream_ = stream;
+    return call_pool(pool_, msg);
+  }
+  // before the stream is waited for, so that the wait gives the memory back to the pool
+  void release() {
+    for (void *p : ptrs_) cudaFreeAsync(p, stream_);
+    ptrs_.clear();
+    left_ = 0;
   }
   template <typename X>
   X *alloc(size_t n, std::string &msg) {
-    void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, n * sizeof(X) > 0 ? n * sizeof(X) : 1);
-    if (e != cudaSuccess) {
-      msg = std::string("device allocation failed: ") + cudaGetErrorString(e);
-      return nullptr;
+    const size_t bytes = (std::max<size_t>(n * sizeof(X), 1) + 255) / 256 * 256;
+    if (bytes > left_) {
+      size_t want = std::max(bytes, CHUNK);
+      void *p = nullptr;
+      cudaError_t e = cudaMallocFromPoolAsync(&p, want, pool_, stream_);
+      if (e == cudaErrorMemoryAllocation && want > bytes) {  // no room for a whole chunk
+        cudaGetLastError();
+        want = bytes;
+        e = cudaMallocFromPoolAsync(&p, want, pool_, stream_);
+      }
+      if (e != cudaSuccess) {
+        msg = std::string("device allocation failed: ") + cudaGetErrorString(e);
+        return nullptr;
+      }
+      ptrs_.push_back(p);
+      if (want == bytes) return static_cast<X *>(p);
+      next_ = static_cast<unsigned char *>(p);
+      left_ = want;
     }
-    ptrs_.push_back(p);
-    return static_cast<X *>(p);
+    X *r = reinterpret_cast<X *>(next_);
+    next_ += bytes;
+    left_ -= bytes;
+    return r;
   }
 
  private:
+  static constexpr size_t CHUNK = (size_t)32 << 20;
+  cudaMemPool_t pool_ = nullptr;
+  cudaStream_t stream_ = nullptr;
   std::vector<void *> ptrs_;
+  unsigned char *next_ = nullptr;
+  size_t left_ = 0;
 };
 
 // Trilinear stencil of lin_stencil (same brackets and clamped fractions) plus, per axis, the
@@ -1382,10 +1444,10 @@ class Adjoint {
   explicit Adjoint(const AdjointProblem &pr) : pr_(pr) {}
   ~Adjoint() {
     if (stream_) {
+      pool_.release();
       cudaStreamSynchronize(stream_);
       cudaStreamDestroy(stream_);
     }
-    if (red_host_) cudaFreeHost(red_host_);
   }
 
   bool run(double *J, std::string &msg) {
@@ -1395,7 +1457,8 @@ class Adjoint {
     if (pr_.gu && pr_.gv && pr_.gw && !backward(msg)) return false;
     ACK(cudaStreamSynchronize(stream_));
     DevReduce r{};
-    ACK(cudaMemcpy(&r, red_dev_, sizeof(DevReduce), cudaMemcpyDeviceToHost));
+    ACK(cudaMemcpyAsync(&r, red_dev_, sizeof(DevReduce), cudaMemcpyDeviceToHost, stream_));
+    ACK(cudaStreamSynchronize(stream_));
     if (r.err) {
       msg = "adjoint: device error in the advection kernels";
       return false;
@@ -1428,6 +1491,8 @@ class Adjoint {
         msg = "adjoint: level times must increase";
         return false;
       }
+    ACK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    if (!pool_.open(stream_, msg)) return false;
     std::vector<int> flag((size_t)n[0] * n[1] * n[2], 0);
     if (pr_.flag) std::memcpy(flag.data(), pr_.flag, flag.size() * sizeof(int));
     if (!hg_.build(n, pr_.x, pr_.y, pr_.z, flag.data())) {
@@ -1483,7 +1548,7 @@ class Adjoint {
       // the padded flags and boundary normals of the grid (the library's make_dev_grid)
       int8_t *f = pool_.alloc<int8_t>(hg_.flag.size(), msg);
       if (!f) return false;
-      ACK(cudaMemcpy(f, hg_.flag.data(), hg_.flag.size(), cudaMemcpyHostToDevice));
+      ACK(cudaMemcpyAsync(f, hg_.flag.data(), hg_.flag.size(), cudaMemcpyHostToDevice, stream_));
       dg_.flag = f;
       for (int a = 0; a < 3; a++) {
         std::vector<lcsdata_t> comp(hg_.ntot(), lcsdata_t(0));
@@ -1517,9 +1582,7 @@ class Adjoint {
         if (!(axT_[a].pull = upload(pullT, msg))) return false;
       }
     }
-    ACK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    ACK(cudaMallocHost(&red_host_, sizeof(DevReduce)));
-    if (!(red_dev_ = pool_.alloc<DevReduce>(1, msg))) return false;
+    if (!(red_dev_ = pool_.alloc<DevReduce>(pr_.nlevels + 1, msg))) return false;
     return true;
   }
 
@@ -1528,7 +1591,8 @@ class Adjoint {
     std::vector<T> tmp(h.begin(), h.end());
     T *d = pool_.alloc<T>(tmp.size(), msg);
     if (!d) return nullptr;
-    if (cudaMemcpy(d, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) {
+    // (pageable source: staged before the call returns)
+    if (cudaMemcpyAsync(d, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice, stream_) != cudaSuccess) {
       msg = "adjoint: upload failed";
       return nullptr;
     }
@@ -1537,11 +1601,12 @@ class Adjoint {
 
   dim3 node_grid() const { return dim3((dg_.P.n[0] + 31) / 32, (dg_.P.n[1] + 7) / 8, dg_.P.n[2]); }
 
+  // three zeroed padded fields, one behind the other
   bool field3(T *f[3], std::string &msg) {
-    for (int c = 0; c < 3; c++) {
-      if (!(f[c] = pool_.alloc<T>(ntot_, msg))) return false;
-      ACK(cudaMemsetAsync(f[c], 0, ntot_ * sizeof(T), stream_));
-    }
+    T *base = pool_.alloc<T>(3 * (size_t)ntot_, msg);
+    if (!base) return false;
+    ACK(cudaMemsetAsync(base, 0, 3 * (size_t)ntot_ * sizeof(T), stream_));
+    for (int c = 0; c < 3; c++) f[c] = base + c * (size_t)ntot_;
     return true;
   }
 
@@ -1584,27 +1649,31 @@ class Adjoint {
     // padded levels + CFL maxima -> subcycles of every update (set_dt, src/lp_motion_m.f90:56-127)
     if (!slab(U_, (size_t)3 * L, msg)) return false;
     cmax_.assign(L, 0.0);
+    std::vector<DevReduce> red(L + 1);
+    const double big = std::numeric_limits<double>::max();
+    for (DevReduce &r : red) {
+      r = DevReduce{};
+      std::memcpy(&r.cmin, &big, sizeof(double));
+    }
+    ACK(cudaMemcpyAsync(red_dev_, red.data(), red.size() * sizeof(DevReduce), cudaMemcpyHostToDevice, stream_));
     for (int l = 0; l < L; l++) {
       T *f[3] = {U_[3 * l], U_[3 * l + 1], U_[3 * l + 2]};
-      DevReduce init{};
-      double big = std::numeric_limits<double>::max();
-      std::memcpy(&init.cmin, &big, sizeof(double));
-      *red_host_ = init;
-      ACK(cudaMemcpyAsync(red_dev_, red_host_, sizeof(DevReduce), cudaMemcpyHostToDevice, stream_));
       if (flags_)
         k_ingest<T, T, lcsdata_t, true><<<node_grid(), dim3(32, 8, 1), 0, stream_>>>(dg_, pr_.u[l], pr_.v[l], pr_.w[l], f[0], f[1], f[2],
-                                                                                   red_dev_);
+                                                                                   red_dev_ + 1 + l);
       else
         k_ingest<T, T, lcsdata_t, false><<<node_grid(), dim3(32, 8, 1), 0, stream_>>>(dg_, pr_.u[l], pr_.v[l], pr_.w[l], f[0], f[1], f[2],
-                                                                                    red_dev_);
+                                                                                    red_dev_ + 1 + l);
       ACK(cudaGetLastError());
-      ACK(cudaMemcpyAsync(red_host_, red_dev_, sizeof(DevReduce), cudaMemcpyDeviceToHost, stream_));
-      ACK(cudaStreamSynchronize(stream_));
-      if (red_host_->err) {
+    }
+    ACK(cudaMemcpyAsync(red.data(), red_dev_, red.size() * sizeof(DevReduce), cudaMemcpyDeviceToHost, stream_));
+    ACK(cudaStreamSynchronize(stream_));
+    for (int l = 0; l < L; l++) {
+      if (red[1 + l].err) {
         msg = "adjoint: non-finite velocity";
         return false;
       }
-      std::memcpy(&cmax_[l], &red_host_->cmax, sizeof(double));
+      std::memcpy(&cmax_[l], &red[1 + l].cmax, sizeof(double));
     }
     nsub_.assign(L, 0);
     for (int l = 1; l < L; l++) {
@@ -1657,8 +1726,7 @@ class Adjoint {
     for (int l = 1; l < L; l++) {
       if ((l - 1) % K == 0) {
         const int s = (l - 1) / K;
-        for (int c = 0; c < 3; c++)
-          ACK(cudaMemcpyAsync(cp_[3 * s + c], fm_[cur_][c], ntot_ * sizeof(T), cudaMemcpyDeviceToDevice, stream_));
+        ACK(cudaMemcpyAsync(cp_[3 * s], fm_[cur_][0], 3 * (size_t)ntot_ * sizeof(T), cudaMemcpyDeviceToDevice, stream_));
       }
       if (!advance(l, fm_, cur_, nullptr, msg, tangent_)) return false;
     }
@@ -1969,7 +2037,7 @@ class Adjoint {
           FieldPtrsW<T> fw{};
           for (int c = 0; c < 3; c++) fw.f[c] = fbar[fb][c];
           fold<GHOST_FM>(fw);
-          for (int c = 0; c < 3; c++) ACK(cudaMemsetAsync(fbar[fb ^ 1][c], 0, ntot_ * sizeof(T), stream_));
+          ACK(cudaMemsetAsync(fbar[fb ^ 1][0], 0, 3 * (size_t)ntot_ * sizeof(T), stream_));
           FieldPtrs<T> fo{}, fbn{};
           FieldPtrsW<T> fbo{};
           for (int c = 0; c < 3; c++) {
@@ -2110,7 +2178,7 @@ class Adjoint {
   DevGrid<T> dg_{};
   Pool pool_;
   cudaStream_t stream_ = nullptr;
-  DevReduce *red_host_ = nullptr, *red_dev_ = nullptr;
+  DevReduce *red_dev_ = nullptr;  // [0]: the sweeps' error word; [1 + l]: ingest of level l
   long N_ = 0, ntot_ = 0;
   std::vector<T *> U_, Ub_, cp_;
   std::vector<double> cmax_;
@@ -2125,6 +2193,12 @@ class Adjoint {
 };
 
 }  // namespace
+
+void adjoint_release_memory() {
+  std::lock_guard<std::mutex> guard(g_pool_lock);
+  for (cudaMemPool_t p : g_pools)
+    if (p) cudaMemPoolTrimTo(p, 0);
+}
 
 bool adjoint_ftle(const AdjointProblem &p, double *J, std::string &msg) {
   Adjoint<lcsdata_t> a(p);

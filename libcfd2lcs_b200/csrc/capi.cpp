@@ -309,6 +309,7 @@ CFD2LCS_EXPORT void cfd2lcs_finalize_(void) {
   if (lib.error) return;
   lib.eng.reset();
   lib.inited = false;
+  cfd2lcs::adjoint_release_memory();
 }
 
 // ----------------------------------------------------------------------- extensions
@@ -336,6 +337,7 @@ CFD2LCS_EXPORT void cfd2lcs_reset_c(void) {
   lib.opt = Options();
   lib.sync_timer = false;
   lib.info = InfoState();
+  cfd2lcs::adjoint_release_memory();
 }
 
 CFD2LCS_EXPORT int cfd2lcs_get_ftle_c(int lcs_handle, lcsdata_t *ftle) {
@@ -648,6 +650,7 @@ CFD2LCS_EXPORT int cfd2lcs_batch_error_c(char *msg, size_t len) {
 CFD2LCS_EXPORT void cfd2lcs_batch_reset_c(void) {
   Batch &b = BT();
   b.inst.clear();
+  cfd2lcs::adjoint_release_memory();
   b.error = 0;
   b.msg.clear();
 }

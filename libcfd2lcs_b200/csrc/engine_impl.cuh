@@ -769,6 +769,8 @@ class Engine : public EngineBase {
       d.have_frame = true;
       if (!d.aux_parent) counters_.ftle_frames++;
     }
+    // the device error word comes back with the update's last event
+    CK(cudaMemcpyAsync(&red_host_->err, &red_->err, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     CK(cudaEventRecord(ev_[9], stream_));
     return true;
   }
@@ -813,7 +815,8 @@ class Engine : public EngineBase {
         return false;
       }
     }
-    return sync_errors(msg);
+    red_err_ |= red_host_->err;
+    return red_err_ ? err_msg(msg) : true;
   }
 
   bool sync_errors(std::string &msg) override {
@@ -909,11 +912,8 @@ class Engine : public EngineBase {
     }
     CK(cudaStreamSynchronize(stream_));
     const long nd = dN(*d);
-    std::vector<T> tmp(nd);
-    for (int c = 0; c < 3; c++) {
-      CK(cudaMemcpy(tmp.data(), d->composed[c], nd * sizeof(T), cudaMemcpyDeviceToHost));
-      for (long q = 0; q < nd; q++) out[c * nd + q] = (lcsdata_t)tmp[q];
-    }
+    static_assert(std::is_same<T, lcsdata_t>::value, "flow maps are kept in the interface type");
+    for (int c = 0; c < 3; c++) CK(cudaMemcpy(out + c * nd, d->composed[c], nd * sizeof(T), cudaMemcpyDeviceToHost));
     return true;
   }
 
