@@ -133,6 +133,45 @@ class Pool {
   size_t left_ = 0;
 };
 
+// Scatters of a warp of nodes that are neighbours along x.  Lane l's stencil starts at padded index
+// p0; where lane l + m's starts m further on (neighbouring nodes mostly move alike), what lane l adds
+// m cells into its row is lane l + m's own first cell, so it is handed over in registers and added
+// there: one atomic per cell and row instead of one per tap.  mask: the lanes that scatter (all of
+// them call).  recv[m-1]: lane l - m hands its m-th tap to this lane; send[m-1]: lane l + m takes
+// this lane's.
+template <int M>
+struct RowLinks {
+  unsigned mask;
+  bool recv[M], send[M];
+};
+
+template <int M>
+__device__ __forceinline__ RowLinks<M> row_links(unsigned mask, int p0) {
+  RowLinks<M> r;
+  r.mask = mask;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int m = 1; m <= M; m++) {
+    const int below = __shfl_up_sync(mask, p0, m), above = __shfl_down_sync(mask, p0, m);
+    r.recv[m - 1] = lane >= m && ((mask >> (lane - m)) & 1u) && below + m == p0;
+    r.send[m - 1] = lane + m < 32 && ((mask >> (lane + m)) & 1u) && above == p0 + m;
+  }
+  return r;
+}
+
+// v[0..M] onto the cells q, q + 1, .. of f (rows of one warp as above)
+template <int M, typename T>
+__device__ __forceinline__ void row_add(const RowLinks<M> &r, T *f, int q, const T (&v)[M + 1]) {
+  T sum = v[0];
+#pragma unroll
+  for (int m = 1; m <= M; m++) {
+    const T w = __shfl_up_sync(r.mask, v[m], m);
+    if (r.recv[m - 1]) sum += w;
+    if (!r.send[m - 1]) atomicAdd(f + q + m, v[m]);
+  }
+  atomicAdd(f + q, sum);
+}
+
 // Trilinear stencil of lin_stencil (same brackets and clamped fractions) plus, per axis, the
 // derivative of the fraction with respect to the coordinate (0 where the fraction is clamped).
 template <typename T>
@@ -233,6 +272,22 @@ __device__ __forceinline__ void bc_adjoint(const DevGrid<T> &g, bool stick, bool
     if (c == sa) xb[c] = T(0);
 }
 
+// the transpose of a trilinear sample around a node: corner q of a gets its weight times ub (the
+// brackets of a node are a cell wide, so the upper x corner is the next cell)
+template <typename T>
+__device__ __forceinline__ void lin_scatter(unsigned mask, const LinStencil<T> &st, FieldPtrsW<T> a, const T ub[3]) {
+  const RowLinks<1> r = row_links<1>(mask, st.p0);
+#pragma unroll
+  for (int q = 0; q < 8; q += 2) {
+    const int cell = st.p0 + ((q & 2) ? st.s[1] : 0) + ((q & 4) ? st.s[2] : 0);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const T v[2] = {st.w[q] * ub[c], st.w[q + 1] * ub[c]};
+      row_add<1>(r, a.f[c], cell, v);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // Adjoint of one backward SL subcycle (k_sl_subcycle with LINEAR interpolation; F: boundary flags).
 // fbn: adjoint of the new flow map (interior values used); fbo: accumulated adjoint of the
@@ -246,10 +301,12 @@ template <typename T, int INTEG, bool F = false>
 __global__ void __launch_bounds__(256) k_sl_adjoint(DevGrid<T> g, VelFields<T> V, FieldPtrs<T> fmo, FieldPtrs<T> fbn, FieldPtrsW<T> fbo,
                                                      FieldPtrsW<T> a1, FieldPtrsW<T> a2, FieldPtrsW<T> a3, StageTimes S, T dt) {
   int i, j, k;
-  if (!node_of_thread(g.P.n, i, j, k)) return;
-  const int p = pidx(g.P.sx, g.P.sxy, i, j, k);
-  const T a[3] = {fbn.f[0][p], fbn.f[1][p], fbn.f[2][p]};
-  if (a[0] == T(0) && a[1] == T(0) && a[2] == T(0)) return;
+  const bool in = node_of_thread(g.P.n, i, j, k);
+  const int p = in ? pidx(g.P.sx, g.P.sxy, i, j, k) : 0;
+  const T a[3] = {in ? fbn.f[0][p] : T(0), in ? fbn.f[1][p] : T(0), in ? fbn.f[2][p] : T(0)};
+  const bool live = in && (a[0] != T(0) || a[1] != T(0) || a[2] != T(0));
+  const unsigned mask = __ballot_sync(0xffffffffu, live);  // the lanes of this row that scatter
+  if (!live) return;
   const T HALF = T(1) / T(2);
   const int no[3] = {i, j, k};
   const T x0[3] = {__ldg(g.lt[0] + i), __ldg(g.lt[1] + j), __ldg(g.lt[2] + k)};
@@ -342,14 +399,13 @@ __global__ void __launch_bounds__(256) k_sl_adjoint(DevGrid<T> g, VelFields<T> V
   lin_stencil_ad(g, x, no, s3);
   // --- fm_new = fm_old(x) + (x - x0) ---
   T xb[3] = {a[0], a[1], a[2]};
+  lin_scatter(mask, s3.st, fbo, a);
 #pragma unroll
   for (int q = 0; q < 8; q++) {
     const int cq = corner(s3.st, q);
-    const T wq = s3.st.w[q];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const T f = __ldg(fmo.f[c] + cq);
-      atomicAdd(fbo.f[c] + cq, wq * a[c]);
 #pragma unroll
       for (int d = 0; d < 3; d++) xb[d] += a[c] * dweight(s3.t, q, d) * s3.dtdx[d] * f;
     }
@@ -361,13 +417,12 @@ __global__ void __launch_bounds__(256) k_sl_adjoint(DevGrid<T> g, VelFields<T> V
   // a, returning the adjoint of the sample position in pb
   auto stage_back = [&](const LinStencilAD<T> &st, const T ub[3], FieldPtrsW<T> a, T omc, T ct, T pb[3]) {
     pb[0] = pb[1] = pb[2] = T(0);
+    lin_scatter(mask, st.st, a, ub);
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       const int cq = corner(st.st, q);
-      const T wq = st.st.w[q];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        atomicAdd(a.f[c] + cq, wq * ub[c]);
         const T vb = omc * __ldg(V.un[c] + cq) + ct * __ldg(V.unp1[c] + cq);
 #pragma unroll
         for (int d = 0; d < 3; d++) pb[d] += ub[c] * dweight(st.t, q, d) * st.dtdx[d] * vb;
@@ -423,13 +478,12 @@ __global__ void __launch_bounds__(256) k_sl_adjoint(DevGrid<T> g, VelFields<T> V
     T u2b[3], xhb[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int c = 0; c < 3; c++) u2b[c] = dt * xb[c];
+    lin_scatter(mask, s2.st, a2, u2b);
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       const int cq = corner(s2.st, q);
-      const T wq = s2.st.w[q];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        atomicAdd(a2.f[c] + cq, wq * u2b[c]);
         const T vb = omc1 * __ldg(V.un[c] + cq) + ct1 * __ldg(V.unp1[c] + cq);
 #pragma unroll
         for (int d = 0; d < 3; d++) xhb[d] += u2b[c] * dweight(s2.t, q, d) * s2.dtdx[d] * vb;
@@ -772,21 +826,23 @@ __device__ __forceinline__ T cubic_value_grad(const DevGrid<T> &g, const CubicSt
   return vz;
 }
 
-// adjoint of the contraction: coefficient q gets its basis product times a[c] (component c)
+// adjoint of the contraction: coefficient q gets its basis product times a[c] (component c); mask:
+// the lanes of the warp's row that scatter this sample
 template <typename T>
-__device__ __forceinline__ void cubic_scatter(const DevGrid<T> &g, const CubicStencil<T> &st, FieldPtrsW<T> C, const T a[3]) {
+__device__ __forceinline__ void cubic_scatter(unsigned mask, const DevGrid<T> &g, const CubicStencil<T> &st, FieldPtrsW<T> C, const T a[3]) {
+  const RowLinks<3> r = row_links<3>(mask, st.p0);
 #pragma unroll
   for (int c2 = 0; c2 < 4; c2++)
 #pragma unroll
     for (int c1 = 0; c1 < 4; c1++) {
       const T w21 = st.b[2][c2] * st.b[1][c1];
+      const int q = st.p0 + c1 * g.P.sx + c2 * g.P.sxy;
 #pragma unroll
-      for (int c0 = 0; c0 < 4; c0++) {
-        const T w = w21 * st.b[0][c0];
-        const int q = st.p0 + c0 + c1 * g.P.sx + c2 * g.P.sxy;
+      for (int c = 0; c < 3; c++) {
+        T v[4];
 #pragma unroll
-        for (int c = 0; c < 3; c++)
-          if (a[c] != T(0)) atomicAdd(C.f[c] + q, w * a[c]);
+        for (int c0 = 0; c0 < 4; c0++) v[c0] = w21 * st.b[0][c0] * a[c];
+        row_add<3>(r, C.f[c], q, v);
       }
     }
 }
@@ -828,10 +884,12 @@ __global__ void __launch_bounds__(128) k_sl_adjoint_cubic(DevGrid<T> g, SplineAx
                                                            FieldPtrs<T> cfm, FieldPtrs<T> fbn, FieldPtrsW<T> cbo, FieldPtrsW<T> a1,
                                                            FieldPtrsW<T> a2, FieldPtrsW<T> a3, StageTimes S, T dt) {
   int i, j, k;
-  if (!node_of_thread(g.P.n, i, j, k)) return;
-  const int p = pidx(g.P.sx, g.P.sxy, i, j, k);
-  const T a[3] = {fbn.f[0][p], fbn.f[1][p], fbn.f[2][p]};
-  if (a[0] == T(0) && a[1] == T(0) && a[2] == T(0)) return;
+  const bool in = node_of_thread(g.P.n, i, j, k);
+  const int p = in ? pidx(g.P.sx, g.P.sxy, i, j, k) : 0;
+  const T a[3] = {in ? fbn.f[0][p] : T(0), in ? fbn.f[1][p] : T(0), in ? fbn.f[2][p] : T(0)};
+  const bool live = in && (a[0] != T(0) || a[1] != T(0) || a[2] != T(0));
+  const unsigned mask = __ballot_sync(0xffffffffu, live);  // the lanes of this row that scatter
+  if (!live) return;
   const T HALF = T(1) / T(2), SIXTH = T(1) / T(6), TWOTHIRD = T(2) / T(3), TWO = T(2);
   const int no[3] = {i, j, k};
   const T x0[3] = {__ldg(g.lt[0] + i), __ldg(g.lt[1] + j), __ldg(g.lt[2] + k)};
@@ -908,8 +966,10 @@ __global__ void __launch_bounds__(128) k_sl_adjoint_cubic(DevGrid<T> g, SplineAx
   T xb[3] = {a[0], a[1], a[2]};
   {
     CubicStencil<T> sf;
-    if (cubic_stencil_d(g, sa, x, no, sf)) {
-      cubic_scatter(g, sf, cbo, a);
+    const bool ok = cubic_stencil_d(g, sa, x, no, sf);
+    const unsigned some = __ballot_sync(mask, ok);
+    if (ok) {
+      cubic_scatter(some, g, sf, cbo, a);
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         T gr[3];
@@ -924,8 +984,9 @@ __global__ void __launch_bounds__(128) k_sl_adjoint_cubic(DevGrid<T> g, SplineAx
   // returning the adjoint of the sample position ---
   auto stage_back = [&](const CubicSample<T> &sm, const T ub[3], FieldPtrsW<T> as, T pb[3]) {
     pb[0] = pb[1] = pb[2] = T(0);
+    const unsigned some = __ballot_sync(mask, sm.ok);
     if (!sm.ok) return;
-    cubic_scatter(g, sm.st, as, ub);
+    cubic_scatter(some, g, sm.st, as, ub);
 #pragma unroll
     for (int c = 0; c < 3; c++)
 #pragma unroll
@@ -1438,6 +1499,22 @@ __global__ void __launch_bounds__(256) k_grad_out(DevGrid<T> g, FieldPtrs<T> src
   gw[q] = src.f[2][p];
 }
 
+// block b's part of sum w f over n values
+template <typename T>
+__global__ void __launch_bounds__(256) k_weighted_sum(const T *__restrict__ w, const T *__restrict__ f, long n, double *__restrict__ part) {
+  double s = 0.0;
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) s += (double)w[q] * (double)f[q];
+  __shared__ double sh[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < 8; q++) s += sh[q];
+    part[blockIdx.x] = s;
+  }
+}
+
 template <typename T>
 class Adjoint {
  public:
@@ -1749,12 +1826,17 @@ class Adjoint {
     if (flags_) k_ftle<T, T, true><<<node_grid(), dim3(32, 8, 1), 0, stream_>>>(dg_, cm, ftle, Tint, 0);
     else k_ftle<T, T, false><<<node_grid(), dim3(32, 8, 1), 0, stream_>>>(dg_, cm, ftle, Tint, 0);
     ACK(cudaGetLastError());
-    std::vector<T> hf(N_), hw(N_);
-    ACK(cudaMemcpyAsync(hf.data(), ftle, N_ * sizeof(T), cudaMemcpyDeviceToHost, stream_));
-    ACK(cudaMemcpyAsync(hw.data(), pr_.weight, N_ * sizeof(T), cudaMemcpyDeviceToHost, stream_));
+    // J = sum weight * FTLE: block sums in FP64, added up in order on the host
+    constexpr int SUM_BLOCKS = 296;
+    double *part = pool_.alloc<double>(SUM_BLOCKS, msg);
+    if (!part) return false;
+    k_weighted_sum<T><<<SUM_BLOCKS, 256, 0, stream_>>>(pr_.weight, ftle, N_, part);
+    ACK(cudaGetLastError());
+    std::vector<double> hp(SUM_BLOCKS);
+    ACK(cudaMemcpyAsync(hp.data(), part, SUM_BLOCKS * sizeof(double), cudaMemcpyDeviceToHost, stream_));
     ACK(cudaStreamSynchronize(stream_));
     double s = 0.0;
-    for (long q = 0; q < N_; q++) s += (double)hw[q] * (double)hf[q];
+    for (double v : hp) s += v;
     *J = s;
     if (tangent_) {
       double *dj = pool_.alloc<double>(N_, msg);
@@ -1777,10 +1859,10 @@ class Adjoint {
   }
 
   // every subcycle of update l (levels l-1 -> l) on the double buffer buf, starting from
-  // buf[cur]; cur follows the result.  With `keep`, the flow map before subcycle q is copied
-  // to keep[3 q + c].
+  // buf[cur]; cur follows the result.  With `keep` instead of buf, from one kept map to the next:
+  // subcycle q takes keep[3 q + c] to keep[3 (q + 1) + c].
   // With `tangent`, the tangent map dfm_ advances alongside (dfm_[cur] pairs with buf[cur]).
-  bool advance(int l, T *buf[2][3], int &cur, T *const *keep, std::string &msg, bool tangent = false) {
+  bool advance(int l, T *(*buf)[3], int &cur, T *const *keep, std::string &msg, bool tangent = false) {
     const lcsdata_t t0 = pr_.times[l - 1], t1 = pr_.times[l];
     const lcsdata_t dt_f = t1 - t0;
     const int ns = nsub_[l];
@@ -1791,10 +1873,16 @@ class Adjoint {
       V.unp1[c] = U_[3 * l + c];
     }
     lcsdata_t lp = t1;
+    T *chain[2][3];
     for (int q = 0; q < ns; q++) {
-      if (keep)
-        for (int c = 0; c < 3; c++)
-          ACK(cudaMemcpyAsync(keep[3 * q + c], buf[cur][c], ntot_ * sizeof(T), cudaMemcpyDeviceToDevice, stream_));
+      if (keep) {
+        cur = 0;
+        buf = chain;
+        for (int c = 0; c < 3; c++) {
+          chain[0][c] = keep[3 * q + c];
+          chain[1][c] = keep[3 * (q + 1) + c];
+        }
+      }
       const StageTimes S = stage_times(t0, t1, lp, dt);
       FieldPtrs<T> fo{};
       FieldPtrsW<T> fn{};
@@ -2000,19 +2088,16 @@ class Adjoint {
       maxsub = std::max(maxsub, m);
     }
     std::vector<T *> states;
-    if (!slab(states, (size_t)3 * maxsub, msg)) return false;
-    T *work[2][3];
-    for (int b = 0; b < 2; b++)
-      for (int c = 0; c < 3; c++) work[b][c] = fm_[b][c];  // the forward buffers are free now
+    if (!slab(states, (size_t)3 * (maxsub + 1), msg)) return false;
     for (int s = nseg - 1; s >= 0; s--) {
       const int l0 = s * K + 1, l1 = std::min((s + 1) * K, L - 1);
       // recompute the segment from its checkpoint, keeping the flow map before each subcycle
       std::vector<int> first(l1 - l0 + 2, 0);
       for (int l = l0; l <= l1; l++) first[l - l0 + 1] = first[l - l0] + nsub_[l];
-      for (int c = 0; c < 3; c++) ACK(cudaMemcpyAsync(work[0][c], cp_[3 * s + c], ntot_ * sizeof(T), cudaMemcpyDeviceToDevice, stream_));
-      int wc = 0;
+      ACK(cudaMemcpyAsync(states[0], cp_[3 * s], 3 * (size_t)ntot_ * sizeof(T), cudaMemcpyDeviceToDevice, stream_));
+      int unused = 0;
       for (int l = l0; l <= l1; l++)
-        if (!advance(l, work, wc, &states[(size_t)3 * first[l - l0]], msg)) return false;
+        if (!advance(l, nullptr, unused, &states[(size_t)3 * first[l - l0]], msg)) return false;
       // reverse through the segment
       for (int l = l1; l >= l0; l--) {
         const lcsdata_t t0 = pr_.times[l - 1], t1 = pr_.times[l];
