@@ -342,7 +342,8 @@ class Engine : public EngineBase {
       if (!(d.P.slot = arena_.alloc<int>(dn, msg))) return false;
       d.P2.slot = d.P.slot;  // the inverse map is rewritten whole by every permutation
       // key space for either tile shape of the sort (gathering or staged forward kernel)
-      const long ncell = std::max(sort_key_space(sort_tiles(n_, 32, SORT_TY, SORT_TZ)), sort_key_space(sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ)));
+      const long ncell = std::max({sort_key_space(gather_tiles(n_, false)), sort_key_space(gather_tiles(n_, true)),
+                                   sort_key_space(sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ))});
       if (ncell > (long)std::numeric_limits<int>::max()) {
         msg = "diagnostic_init: grid too large for the forward particle sort";
         return false;
@@ -401,7 +402,7 @@ class Engine : public EngineBase {
     }
     if (!(cp_[0].slot = arena_.alloc<int>(N_, msg))) return false;
     cp_[1].slot = cp_[0].slot;
-    const long ncell = sort_key_space(sort_tiles(n_, 32, SORT_TY, SORT_TZ));
+    const long ncell = std::max(sort_key_space(gather_tiles(n_, false)), sort_key_space(gather_tiles(n_, true)));
     if (ncell > (long)std::numeric_limits<int>::max()) {
       msg = "diagnostic_init: grid too large for the composition sort";
       return false;
@@ -645,11 +646,12 @@ class Engine : public EngineBase {
         } else {
           // the variant holds from one sort to the next (the staged kernel reads the sort's tiles)
           const bool usable = fwd_tile_usable(iv, V);
-          // the staged family re-sorts every kSortInterval subcycles of the update (its tiles
-          // must be the sort's); the gathering-only sets re-sort when their launches have lost
+          // the staged family re-sorts at an interval (the staged form's tiles must be the sort's, so
+          // after a reset the set gathers until its next sort); the gathering-only sets re-sort when their launches have lost
           // more time to disorder than a sort costs (sort_due)
           const int di = (int)(&d - diags_.data());
-          const bool resort = usable ? sc % sort_interval(interp) == 0 : sort_due(d);
+          const bool resort =
+              usable ? d.since_sort >= sort_interval(d) || (tile_mode_ == 2 && d.fwd_variant != 1) : sort_due(d);
           if (resort) {
             d.fwd_variant = usable ? tile_variant(1) : 0;
             if (!usable) {
@@ -1973,7 +1975,7 @@ class Engine : public EngineBase {
   void compose_steps(const SplineAxes<T> &sa, DiagT &d, int m, FieldPtrsW<T> out) {
     const int np = (int)N_, grd = (np + 255) / 256;
     int *err = &red_->err;
-    const SortTiles st = sort_tiles(n_, 32, SORT_TY, SORT_TZ);
+    const SortTiles st = gather_tiles(n_, interp_is_spline(I));
     std::string dummy;
     k_reset_particles<T><<<node_grid(), dim3(32, 8, 1), 0, stream_>>>(dg_, cp_[0]);
     counters_.kernel_launches++;
@@ -2273,6 +2275,7 @@ class Engine : public EngineBase {
     const dim3 blk(32, 8, 1);
     counters_.kernel_launches++;
     d.since_sort = 0;  // the particles are back on their nodes, in node order
+    d.fwd_variant = 0;  // which is not the staged kernel's
     d.base_ms = -1;
     d.excess_ms = 0;
     if (d.lg) {
@@ -2285,7 +2288,7 @@ class Engine : public EngineBase {
     }
   }
 
-  // Re-sorts the particle slots by grid cell (32 x 4 x 2 tiles, x fastest) every kSortInterval
+  // Re-sorts the particle slots by grid cell (gather_tiles, x fastest) every kSortInterval
   // subcycles, so that the particles of a block gather neighbouring spline taps as the SL
   // kernel's blocks do.  Results do not depend on the order: every particle is advanced
   // independently and the snapshot reads it back through the inverse map.  Measured on B200
@@ -2295,8 +2298,12 @@ class Engine : public EngineBase {
 #define CFD2LCS_SORT_INTERVAL 2
 #endif
   static constexpr int kSortInterval = CFD2LCS_SORT_INTERVAL;
+  // The gathering B-spline kernel in the long rows of gather_tiles: every 1 / 2 / 3 / 4 subcycles
+  // 244.0 / 253.1 / 258.1 / 260.1 ms of launches per pass of 51 at ABC 256^3, and 0.8 ms a sort:
+  // 556 / 546 / 543 / 543 ms per pass in all.
+  static constexpr int kGatherSortInterval = 4;
   int sort_every_ = 0;  // CFD2LCS_B200_SORT_EVERY at cfd2lcs_init (0: the default below)
-  int sort_interval(int interp) const { return sort_every_ > 0 ? sort_every_ : kSortInterval; }
+  long sort_interval(const DiagT &d) const { return sort_every_ > 0 ? sort_every_ : (d.fwd_variant == 1 ? kSortInterval : kGatherSortInterval); }
   // Re-sort schedule of a set whose forward kernel gathers (not the staged family): a sort
   // restores the coalescing the launches lose as the particles drift from the order of the
   // last sort, so it pays once the time they have lost since that sort -- each launch's event
@@ -2333,10 +2340,10 @@ class Engine : public EngineBase {
     d.excess_ms = 0;
     return true;
   }
-  // fwd_tile: the 16 x 4 x 4-cell tiles the staged forward kernel reads, else the 32 x 4 x 2
-  // tiles that suit the gathering kernel
+  // fwd_tile: the 16 x 4 x 4-cell tiles the staged forward kernel reads, else the tiles that suit the
+  // gathering kernel
   bool sort_particles(DiagT &d, std::string &msg, bool fwd_tile = false) {
-    d.sort_geom = fwd_tile ? sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ) : sort_tiles(n_, 32, SORT_TY, SORT_TZ);
+    d.sort_geom = fwd_tile ? sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ) : gather_tiles(n_, opt_->interpolator == QUADRATIC || opt_->interpolator == CUBIC);
     if (!sort_slots(d.P, d.P2, d.pkey, d.pcnt, d.poffs, d.ptsum, (int)dN(d), d.sort_geom, msg)) return false;
     std::swap(d.P, d.P2);
     return true;

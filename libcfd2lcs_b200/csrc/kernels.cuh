@@ -862,12 +862,8 @@ __global__ void k_reset_particles(DevGrid<T> g, Particles<T> P) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Counting sort of the forward particle slots by grid cell: tiles of 32 (x) x 4 (y) x 2 (z)
-// cells, x fastest inside a tile.  A block of 256 particles then covers about one such tile,
-// so its warps share the y and z spline rows the way the backward kernel's blocks do (L1
-// reuse across the block), and each warp walks along x.  Measured on B200 (ABC 256^3 CUBIC,
-// forward launch): tiles 32 x 8 x 1 / 32 x 4 x 2 / 32 x 2 x 4 took 6.91 / 6.72 / 6.82 ms (FP64
-// velocity) and 4.20 / 4.06 / 4.12 ms (FP32).  Steps: count per cell key, exclusive scan of the counts in chunks of
+// Counting sort of the forward particle slots by grid cell: tiles of long rows (gather_tiles), x
+// fastest inside a tile.  Steps: count per cell key, exclusive scan of the counts in chunks of
 // SORT_TILE, and a scatter that moves every particle to its key's next free slot.  Particles
 // of one cell land in arbitrary order, which no result depends on.  The count array returns
 // to zero inside the scan, ready for the next sort.
@@ -875,14 +871,9 @@ __global__ void k_reset_particles(DevGrid<T> g, Particles<T> P) {
 constexpr int SORT_TILE = 2048;  // 256 threads x 8 counts
 
 // Cell tiles of the order: tx x ty x tz cells (tx ty tz = 256), x fastest inside a tile and
-// tiles in x, y, z order; cells c_a in 0..n_a per axis, padded to whole tiles.  The gathering
-// forward kernel takes 32 x 4 x 2 (32 x 8/SORT_TZ x SORT_TZ; measured on B200, see the engine),
-// the staged forward kernel 16 x 4 x 4 (its shared-memory box is that tile widened by 4 cells).
-#ifndef CFD2LCS_SORT_TZ
-#define CFD2LCS_SORT_TZ 2
-#endif
-constexpr int SORT_TZ = CFD2LCS_SORT_TZ, SORT_TY = 8 / SORT_TZ;
-
+// tiles in x, y, z order; cells c_a in 0..n_a per axis, padded to whole tiles.  The staged forward
+// kernel takes 16 x 4 x 4 (its shared-memory box is that tile widened by 4 cells), the gathering
+// kernels gather_tiles.
 struct SortTiles {
   int tx, ty, tz;     // cells per tile along each axis
   int ntx, nty, ntz;  // tiles along each axis
@@ -897,6 +888,19 @@ __host__ __device__ inline SortTiles sort_tiles(const int n[3], int tx, int ty, 
   s.nty = (n[1] + 1 + ty - 1) / ty;
   s.ntz = (n[2] + 1 + tz - 1) / tz;
   return s;
+}
+
+// The gathering kernels' tiles.  B-splines: rows of up to 128 cells, two deep in y.  About one particle
+// lies in a cell, so a warp spans some 32 cells of the order, and every row it crosses into costs
+// its 64 taps another one or two L1 lines per request: long rows are crossed rarely, and that
+// matters more than the rows a block shares in y and z.  Measured on B200 (ABC 256^3 CUBIC FP64,
+// forward launch, sorted every 2): 32 x 4 x 2 5.24 ms, 64 x 2 x 2 5.08, 64 x 4 x 1 5.04, 128 x 2 x 1
+// 4.96, 256 x 1 x 1 4.91, 16 x 8 x 2 5.53; 101 x 75 x 50: 143 us, 128 x 2 x 1 133.  The 8 taps of
+// the others have the larger share of their lines in y and z: 32 x 4 x 2 (200^3 turbulence in FP32
+// 96.4 ms per pass, 128 x 2 x 1 100.0; ABC 256^3 FP64 even).
+__host__ __device__ inline SortTiles gather_tiles(const int n[3], bool spline) {
+  const int tx = !spline || n[0] < 48 ? 32 : (n[0] < 96 ? 64 : 128);
+  return sort_tiles(n, tx, spline ? 256 / tx : 4, spline ? 1 : 2);
 }
 
 __host__ __device__ inline long sort_key_space(const SortTiles &s) { return (long)s.ntz * s.nty * s.ntx * 256; }
