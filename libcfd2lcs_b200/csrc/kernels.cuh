@@ -134,13 +134,19 @@ __global__ void __launch_bounds__(256) k_ingest(DevGrid<T> g, const U *__restric
 #ifndef CFD2LCS_FWD_MINB_SPLINE
 #define CFD2LCS_FWD_MINB_SPLINE 4
 #endif
+// FP32 positions need half the registers: the LINEAR forward kernel, bound by the latency of its
+// gathers, runs 6 blocks (200^3 turbulence, single library: 4 / 6 / 8 blocks 404 / 353 / 376 us per
+// launch; its B-spline form 641 / 663 / 672 at 150^3, which keeps 4).
+#ifndef CFD2LCS_FWD_MINB_LINEAR_SP
+#define CFD2LCS_FWD_MINB_LINEAR_SP 6
+#endif
 template <int INTERP>
 constexpr int sl_min_blocks() {
   return interp_is_spline(INTERP) ? CFD2LCS_SL_MINB_SPLINE : CFD2LCS_SL_MINB_LINEAR;
 }
-template <int INTERP>
+template <typename T, int INTERP>
 constexpr int fwd_min_blocks() {
-  return interp_is_spline(INTERP) ? CFD2LCS_FWD_MINB_SPLINE : CFD2LCS_FWD_MINB_LINEAR;
+  return interp_is_spline(INTERP) ? CFD2LCS_FWD_MINB_SPLINE : (sizeof(T) == 4 ? CFD2LCS_FWD_MINB_LINEAR_SP : CFD2LCS_FWD_MINB_LINEAR);
 }
 
 template <typename T, typename TV, int INTEG, int INTERP, bool HAS_FLAGS>
@@ -357,7 +363,7 @@ __device__ __forceinline__ void fwd_advance(const DevGrid<T> &g, const SplineAxe
 }
 
 template <typename T, typename TV, int INTEG, int INTERP, bool HAS_FLAGS>
-__global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_subcycle(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P, StageTimes S,
+__global__ void __launch_bounds__(256, fwd_min_blocks<T, INTERP>()) k_fwd_subcycle(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P, StageTimes S,
                                                        T dt, int np, int *err) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= np) return;
@@ -378,7 +384,7 @@ __global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_subcycle(
 // stages read the two velocity levels themselves (no blend fields to write between subcycles).
 // A particle depends on no other, so nothing has to meet between the subcycles.
 template <typename T, typename TV, int INTEG, int INTERP, bool HAS_FLAGS>
-__global__ void __launch_bounds__(256, fwd_min_blocks<INTERP>()) k_fwd_run(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P,
+__global__ void __launch_bounds__(256, fwd_min_blocks<T, INTERP>()) k_fwd_run(DevGrid<T> g, SplineAxes<T> sa, VelFields<TV> V, Particles<T> P,
                                                   const __grid_constant__ StageRun R, T dt, int np, int *err) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= np) return;
@@ -1040,10 +1046,11 @@ struct Pair<float> {
   using type = float2;
 };
 
+constexpr int BLEND_OUT = 6;  // blends written in one pass over the two levels
 template <typename T>
 struct BlendOut {
-  T *f[3][3];  // [output][component]
-  T omc[3], ct[3];
+  T *f[BLEND_OUT][3];  // [output][component]
+  T omc[BLEND_OUT], ct[BLEND_OUT];
 };
 
 template <typename T>
