@@ -663,12 +663,11 @@ __device__ __forceinline__ bool track_pass_lines(const DevGrid<T> &g, const T x[
         q[a][o + 1] = mul_rn(d, d);
       }
     int off[3];
-    if (nbr_scan_short(q, sa, off)) {
-      no[0] += off[0];
-      no[1] += off[1];
-      no[2] += off[2];
-      return off[0] != 0 || off[1] != 0 || off[2] != 0;
-    }
+    nbr_scan_short(q, sa, off);
+    no[0] += off[0];
+    no[1] += off[1];
+    no[2] += off[2];
+    return off[0] != 0 || off[1] != 0 || off[2] != 0;
   }
   T sqp[3][3], sqn[3][3];
   unsigned ok = 0;  // bit 3a+o+1: line no[a]+o is interior, or axis a is periodic

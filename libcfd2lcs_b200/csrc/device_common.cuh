@@ -53,6 +53,8 @@ struct DevGrid {
   const T *li[3];        // interpolation lines, index 0..n+1
   // RN(1 / (li[a][i+1] - li[a][i])), index 0..n: the LINEAR stencils' fractions (lin_quotient)
   const T *ri[3] = {nullptr, nullptr, nullptr};
+  // RN(1 / (bb[a + 3] - bb[a])) of the bounding box, for the composition's node guess (lin_quotient)
+  T bbr[3] = {T(0), T(0), T(0)};
   const T *invd[3];      // inverse half spans, see HostGrid::invd
   const int8_t *flag;    // padded bcflag or nullptr
   const T *nrm[3];       // boundary normals (padded) or nullptr

@@ -1634,6 +1634,7 @@ class Engine : public EngineBase {
     P.single_axis = H.single_axis;
     P.zquirk = H.zquirk;
     for (int q = 0; q < 6; q++) P.bb[q] = (T)H.bb[q];
+    for (int a = 0; a < 3; a++) dg.bbr[a] = T(1) / (P.bb[a + 3] - P.bb[a]);
     for (int d = 0; d < 27; d++)
       for (int c = 0; c < 3; c++) P.ps[d][c] = (T)H.ps[d][c];
     P.has_flags = H.has_flags;

@@ -472,7 +472,7 @@ __device__ __forceinline__ void alltoall_wrap(const DevGrid<T> &g, T x[3], int n
   } else {
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      const T s = clamp01((x[a] - bb[a]) / (bb[a + 3] - bb[a]));
+      const T s = clamp01(lin_quotient(x[a] - bb[a], bb[a + 3] - bb[a], g.bbr[a]));
       const int v = (int)round(T(g.P.n[a]) * s);  // nint(real(n)*s): half away from zero
       no[a] = min(max(v, 1), g.P.n[a]);
     }
