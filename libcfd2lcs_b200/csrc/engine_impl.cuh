@@ -2020,8 +2020,8 @@ class Engine : public EngineBase {
     int *err = &red_->err;
     const SortTiles st = gather_tiles(n_, interp_is_spline(I));
     std::string dummy;
-    k_reset_particles<T><<<node_grid(), dim3(32, 8, 1), 0, stream_>>>(dg_, cp_[0]);
-    counters_.kernel_launches++;
+    if (m == 0)  // no sub-map yet: no displacement
+      for (int c = 0; c < 3; c++) cudaMemsetAsync(out.f[c], 0, np * sizeof(T), stream_);
     int cur = 0;
     for (int s = 0; s < m; s++) {
       if (s > 0 && s % compose_sort_every_ == 0) {
@@ -2030,12 +2030,11 @@ class Engine : public EngineBase {
       }
       FieldPtrs<T> f{};
       for (int c = 0; c < 3; c++) f.f[c] = d.slot_list_host[3 * s + c];
-      if (compose_minb_ == 4) k_compose_step<T, I, FL, COMPOSE_MINB<T>><<<grd, 256, 0, stream_>>>(dg_, sa, f, cp_[cur], np, err);
-      else k_compose_step<T, I, FL, 2><<<grd, 256, 0, stream_>>>(dg_, sa, f, cp_[cur], np, err);
+      const int first = s == 0, last = s == m - 1;
+      if (compose_minb_ == 4) k_compose_step<T, I, FL, COMPOSE_MINB<T>><<<grd, 256, 0, stream_>>>(dg_, sa, f, cp_[cur], np, first, last, out, err);
+      else k_compose_step<T, I, FL, 2><<<grd, 256, 0, stream_>>>(dg_, sa, f, cp_[cur], np, first, last, out, err);
       counters_.kernel_launches++;
     }
-    k_compose_finish<T, FL><<<grd, 256, 0, stream_>>>(dg_, cp_[cur], out, np);
-    counters_.kernel_launches++;
   }
 
   bool launch_compose(int iv, const SplineAxes<T> &sa, DiagT &d, int m, std::string &msg) {

@@ -99,9 +99,13 @@ __global__ void __launch_bounds__(256) k_ingest(DevGrid<T> g, const U *__restric
       cmax = fmax(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
       cmin = fmin(cmin, __shfl_xor_sync(0xffffffffu, cmin, o));
     }
+    // a block whose extremes do not pass what is there already leaves it alone (a stale value only
+    // costs an atomic that changes nothing): one address takes the atomics of every block otherwise,
+    // 221,000 of them at 384^3 (the kernel 733 -> 670 us)
     if (lane == 0) {
-      atomicMax(&red->cmax, (unsigned long long)__double_as_longlong(cmax));
-      atomicMin(&red->cmin, (unsigned long long)__double_as_longlong(cmin));
+      const unsigned long long hi = (unsigned long long)__double_as_longlong(cmax), lo = (unsigned long long)__double_as_longlong(cmin);
+      if (hi > *(volatile unsigned long long *)&red->cmax) atomicMax(&red->cmax, hi);
+      if (lo < *(volatile unsigned long long *)&red->cmin) atomicMin(&red->cmin, lo);
     }
   }
 }
@@ -527,16 +531,30 @@ __global__ void __launch_bounds__(256) k_compose(DevGrid<T> g, SplineAxes<T> sa,
 // one step gather neighbouring taps -- after a few sub-maps the particles of neighbouring nodes
 // are far apart and the node-ordered k_compose gathers each tap sector from HBM.  The per-point
 // sequence is k_compose's loop body, the state kept exactly between steps, so the composed map
-// is bitwise k_compose's.  k_reset_particles starts the particles at their nodes.
+// is bitwise k_compose's.  The first step starts the particles at their nodes, the last one writes the
+// composed map in node order (exchange_lpmap, after the interior flow-map BC) instead of their state:
+// passes of their own for the two were 0.16 ms each at 256^3 and moved the state once more.
 // MINB: resident blocks of 256 threads per SM asked of the compiler (register cap 65536 / (256 MINB))
 template <typename T, int INTERP, bool HAS_FLAGS, int MINB = 2>
-__global__ void __launch_bounds__(256, MINB) k_compose_step(DevGrid<T> g, SplineAxes<T> sa, FieldPtrs<T> f, Particles<T> P, int np, int *err) {
+__global__ void __launch_bounds__(256, MINB) k_compose_step(DevGrid<T> g, SplineAxes<T> sa, FieldPtrs<T> f, Particles<T> P, int np, int first, int last,
+                                                            FieldPtrsW<T> out, int *err) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= np) return;
-  T x[3] = {P.x[0][q], P.x[1][q], P.x[2][q]};
-  int no[3] = {P.no[0][q], P.no[1][q], P.no[2][q]};
-  T d[3] = {P.dx[0][q], P.dx[1][q], P.dx[2][q]};
   constexpr bool CURV = interp_is_curv(INTERP);
+  T x[3], d[3];
+  int no[3];
+  if (first) {
+    no[0] = q % g.P.n[0] + 1, no[1] = (q / g.P.n[0]) % g.P.n[1] + 1, no[2] = q / (g.P.n[0] * g.P.n[1]) + 1;
+    node_xyz<T, CURV>(g, no[0], no[1], no[2], x);
+    d[0] = d[1] = d[2] = T(0);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      x[c] = P.x[c][q];
+      no[c] = P.no[c][q];
+      d[c] = P.dx[c][q];
+    }
+  }
   project_plane<T, CURV>(g, no, x);
   particle_bc<T, HAS_FLAGS, CURV>(g, no, x, err);
   T up[3];
@@ -545,6 +563,17 @@ __global__ void __launch_bounds__(256, MINB) k_compose_step(DevGrid<T> g, Spline
   for (int c = 0; c < 3; c++) {
     x[c] = x[c] + up[c];
     d[c] = d[c] + up[c];
+  }
+  if (last) {
+    const int id = first ? q : P.id[q];
+    bool zero = false;
+    if (HAS_FLAGS) {
+      const int i = id % g.P.n[0] + 1, j = (id / g.P.n[0]) % g.P.n[1] + 1, k = id / (g.P.n[0] * g.P.n[1]) + 1;
+      const int fl = (int)g.flag[pidx(g.P.sx, g.P.sxy, i, j, k)];
+      zero = fl == LCS_MASK || fl == LCS_INFLOW || fl == LCS_OUTFLOW;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) out.f[c][id] = zero ? T(0) : d[c];
   }
   alltoall_wrap<T, CURV>(g, x, no);
   int passes = 0;
@@ -558,28 +587,14 @@ __global__ void __launch_bounds__(256, MINB) k_compose_step(DevGrid<T> g, Spline
     wrap_particle(g, x, no);
     if (!moved) break;
   }
+  if (last) return;
+  if (first) P.id[q] = q;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     P.x[c][q] = x[c];
     P.no[c][q] = no[c];
     P.dx[c][q] = d[c];
   }
-}
-
-// the composed map in node order (exchange_lpmap), after the interior flow-map BC
-template <typename T, bool HAS_FLAGS>
-__global__ void __launch_bounds__(256) k_compose_finish(DevGrid<T> g, Particles<T> P, FieldPtrsW<T> out, int np) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= np) return;
-  const int id = P.id[q];
-  bool zero = false;
-  if (HAS_FLAGS) {
-    const int i = id % g.P.n[0] + 1, j = (id / g.P.n[0]) % g.P.n[1] + 1, k = id / (g.P.n[0] * g.P.n[1]) + 1;
-    const int fl = (int)g.flag[pidx(g.P.sx, g.P.sxy, i, j, k)];
-    zero = fl == LCS_MASK || fl == LCS_INFLOW || fl == LCS_OUTFLOW;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++) out.f[c][id] = zero ? T(0) : P.dx[c][q];
 }
 
 // ---------------------------------------------------------------------------------------
