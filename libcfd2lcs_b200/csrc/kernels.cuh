@@ -1259,26 +1259,35 @@ __host__ __device__ constexpr int fitb_pitch() {
   return XPASS ? LINES + 1 : LINES;
 }
 
+// The factors a sweep reads: the pull table, and for chunks of several lines' worth per warp (LINES <
+// 32) the interior rows' three factors in shared memory: there a warp sweeps several chunks at once,
+// and each would touch a table line of its own with every load.
+template <typename T>
+struct FitCoef {
+  const T *__restrict__ pc;
+  const T *lower, *upper, *pivot;
+};
+
 // One element: the sweeps of pull_forward / pull_backward, or the transposed ones (ADJ).  MID: a
 // row whose second and third off-diagonal factors are zero (every interior row: at its knot a
-// cubic's collocation row has three entries).
-template <typename T, int K, bool FWD, bool ADJ, bool MID>
-__device__ __forceinline__ T fit_step(const T *__restrict__ pc, int i0, T b, T (&win)[3]) {
+// cubic's collocation row has three entries).  SM: those rows' factors from shared memory.
+template <typename T, int K, bool FWD, bool ADJ, bool MID, bool SM>
+__device__ __forceinline__ T fit_step(const FitCoef<T> &C, int i0, T b, T (&win)[3]) {
   if constexpr (MID) {
-    const T *c = pc + 8 * i0;
-    b = b - win[0] * __ldg(c + (FWD ? 0 : 3));
-    if (FWD == ADJ) b = b * __ldg(c + 6);
+    const T *c = C.pc + 8 * i0;
+    b = b - win[0] * (SM ? (FWD ? C.lower[i0] : C.upper[i0]) : __ldg(c + (FWD ? 0 : 3)));
+    if (FWD == ADJ) b = b * (SM ? C.pivot[i0] : __ldg(c + 6));
     win[2] = win[1];
     win[1] = win[0];
     win[0] = b;
     return b;
   } else if constexpr (!ADJ) {
-    if constexpr (FWD) return pull_forward<T, K>(pc, i0, b, win);
-    else return pull_backward<T, K>(pc, i0, b, win);
+    if constexpr (FWD) return pull_forward<T, K>(C.pc, i0, b, win);
+    else return pull_backward<T, K>(C.pc, i0, b, win);
   } else {
-    const T *c = pc + 8 * i0 + (FWD ? 0 : 3);
+    const T *c = C.pc + 8 * i0 + (FWD ? 0 : 3);
     b = b - win[0] * __ldg(c) - win[1] * __ldg(c + 1) - win[2] * __ldg(c + 2);
-    if (FWD) b = b * __ldg(pc + 8 * i0 + 6);
+    if (FWD) b = b * __ldg(C.pc + 8 * i0 + 6);
     win[2] = win[1];
     win[1] = win[0];
     win[0] = b;
@@ -1288,8 +1297,8 @@ __device__ __forceinline__ T fit_step(const T *__restrict__ pc, int i0, T b, T (
 
 // the elements [a, b) of a staged column (from: the values read, to: where they are kept, when
 // STORE) in sweep order
-template <typename T, int K, bool FWD, bool ADJ, bool MID, bool STORE>
-__device__ __forceinline__ void fit_run(const T *__restrict__ pc, const T *from, long fp, T *to, int tp, int a, int b, T (&win)[3]) {
+template <typename T, int K, bool FWD, bool ADJ, bool MID, bool SM, bool STORE>
+__device__ __forceinline__ void fit_run(const FitCoef<T> &C, const T *from, long fp, T *to, int tp, int a, int b, T (&win)[3]) {
   constexpr int G = 4;
   const int step = FWD ? 1 : -1;
   int e = FWD ? a : b - 1;
@@ -1299,32 +1308,41 @@ __device__ __forceinline__ void fit_run(const T *__restrict__ pc, const T *from,
 #pragma unroll
     for (int q = 0; q < G; q++) v[q] = from[(e + q * step) * fp];
 #pragma unroll
-    for (int q = 0; q < G; q++) v[q] = fit_step<T, K, FWD, ADJ, MID>(pc, e + q * step, v[q], win);
+    for (int q = 0; q < G; q++) v[q] = fit_step<T, K, FWD, ADJ, MID, SM>(C, e + q * step, v[q], win);
     if (STORE) {
 #pragma unroll
       for (int q = 0; q < G; q++) to[(e + q * step) * tp] = v[q];
     }
   }
   for (; left > 0; left--, e += step) {
-    const T v = fit_step<T, K, FWD, ADJ, MID>(pc, e, from[e * fp], win);
+    const T v = fit_step<T, K, FWD, ADJ, MID, SM>(C, e, from[e * fp], win);
     if (STORE) to[e * tp] = v;
   }
 }
 
 // [a, b) split into the rows before, in and after [m0, m1), the rows with one off-diagonal factor
-template <typename T, int K, bool FWD, bool ADJ, bool STORE>
-__device__ __forceinline__ void fit_sweep(const T *__restrict__ pc, const T *from, long fp, T *to, int tp, int a, int b, int m0, int m1,
+template <typename T, int K, bool FWD, bool ADJ, bool SM, bool STORE>
+__device__ __forceinline__ void fit_sweep(const FitCoef<T> &C, const T *from, long fp, T *to, int tp, int a, int b, int m0, int m1,
                                           T (&win)[3]) {
   const int p = min(max(m0, a), b), q = min(max(m1, p), b);
   if (FWD) {
-    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, a, p, win);
-    fit_run<T, K, FWD, ADJ, true, STORE>(pc, from, fp, to, tp, p, q, win);
-    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, q, b, win);
+    fit_run<T, K, FWD, ADJ, false, SM, STORE>(C, from, fp, to, tp, a, p, win);
+    fit_run<T, K, FWD, ADJ, true, SM, STORE>(C, from, fp, to, tp, p, q, win);
+    fit_run<T, K, FWD, ADJ, false, SM, STORE>(C, from, fp, to, tp, q, b, win);
   } else {
-    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, q, b, win);
-    fit_run<T, K, FWD, ADJ, true, STORE>(pc, from, fp, to, tp, p, q, win);
-    fit_run<T, K, FWD, ADJ, false, STORE>(pc, from, fp, to, tp, a, p, win);
+    fit_run<T, K, FWD, ADJ, false, SM, STORE>(C, from, fp, to, tp, q, b, win);
+    fit_run<T, K, FWD, ADJ, true, SM, STORE>(C, from, fp, to, tp, p, q, win);
+    fit_run<T, K, FWD, ADJ, false, SM, STORE>(C, from, fp, to, tp, a, p, win);
   }
+}
+
+// elements per chunk: an even share of the line, lengthened for 8 lines so that the two chunks half
+// a warp sweeps sit in different shared-memory banks
+template <bool XPASS, int LINES>
+__host__ __device__ inline int fitb_chunk(int n) {
+  const int ch = (n + FITB_THREADS / LINES - 1) / (FITB_THREADS / LINES);
+  if (LINES != 8) return ch;
+  return XPASS ? (ch + 7) / 16 * 16 + 8 : (ch | 1);
 }
 
 // bitwise comparison (a NaN equals itself)
@@ -1360,19 +1378,29 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
     for (int e = ck; e < n; e += NCH) cp_async_elem(tile + e * P + ln, p + (long)e * es);
   }
   cp_async_commit();
+  constexpr bool SM = LINES < 32;
+  T *const coef = tile + (size_t)n * P;
+  if (SM) {
+    for (int e = threadIdx.x; e < n; e += FITB_THREADS) {
+      coef[e] = __ldg(pc + 8 * e);
+      coef[n + e] = __ldg(pc + 8 * e + 3);
+      coef[2 * n + e] = __ldg(pc + 8 * e + 6);
+    }
+  }
+  const FitCoef<T> C{pc, coef, coef + n, coef + 2 * n};
   cp_async_wait<0>();
   __syncthreads();
-  const int ch = (n + NCH - 1) / NCH;
+  const int ch = fitb_chunk<XPASS, LINES>(n);
   const int c0 = min(ck * ch, n), c1 = min(c0 + ch, n);
   const bool some = c0 < c1;
   T *const col = tile + ln;
   T wf[3] = {T(0), T(0), T(0)}, win[3];
   // --- forward ---
-  if (some) fit_sweep<T, K, true, ADJ, false>(pc, col, P, col, P, max(c0 - warm, 0), c0, m0, m1, wf);
+  if (some) fit_sweep<T, K, true, ADJ, SM, false>(C, col, P, col, P, max(c0 - warm, 0), c0, m0, m1, wf);
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 3; q++) win[q] = wf[q];
-  fit_sweep<T, K, true, ADJ, true>(pc, col, P, col, P, c0, c1, m0, m1, win);
+  fit_sweep<T, K, true, ADJ, SM, true>(C, col, P, col, P, c0, c1, m0, m1, win);
   __syncthreads();
   // the window this chunk has to start from: the last values of the chunk before it
   auto before = [&](T (&w)[3]) {
@@ -1397,7 +1425,7 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
         if (differs(win, wf)) {
 #pragma unroll
           for (int q = 0; q < 3; q++) wf[q] = win[q];
-          fit_sweep<T, K, true, ADJ, true>(pc, s + off, ep, col, P, c0, c1, m0, m1, win);
+          fit_sweep<T, K, true, ADJ, SM, true>(C, s + off, ep, col, P, c0, c1, m0, m1, win);
         }
       }
       __syncthreads();
@@ -1405,11 +1433,11 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
   }
   // --- backward ---
   T wb[3] = {T(0), T(0), T(0)};
-  if (some) fit_sweep<T, K, false, ADJ, false>(pc, col, P, col, P, c1, min(c1 + warm, n), m0, m1, wb);
+  if (some) fit_sweep<T, K, false, ADJ, SM, false>(C, col, P, col, P, c1, min(c1 + warm, n), m0, m1, wb);
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 3; q++) win[q] = wb[q];
-  fit_sweep<T, K, false, ADJ, true>(pc, col, P, col, P, c0, c1, m0, m1, win);
+  fit_sweep<T, K, false, ADJ, SM, true>(C, col, P, col, P, c0, c1, m0, m1, win);
   __syncthreads();
   behind(win);
   if (__syncthreads_or(some && c1 < n && differs(win, wb))) {
@@ -1418,8 +1446,8 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
         behind(win);
         if (differs(win, wb)) {
           // the chunk's forward values again (the source is still whole), then backward
-          fit_sweep<T, K, true, ADJ, true>(pc, s + off, ep, col, P, c0, c1, m0, m1, wf);
-          fit_sweep<T, K, false, ADJ, true>(pc, col, P, col, P, c0, c1, m0, m1, win);
+          fit_sweep<T, K, true, ADJ, SM, true>(C, s + off, ep, col, P, c0, c1, m0, m1, wf);
+          fit_sweep<T, K, false, ADJ, SM, true>(C, col, P, col, P, c0, c1, m0, m1, win);
         }
       }
       __syncthreads();
@@ -1437,24 +1465,29 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
   }
 }
 
-// Lines per block of k_fit_block on an axis of n elements: 32 while two blocks fit an SM, then 16
-// and 8; 0 where the whole-line sweeps run: longer lines, factors that decay too slowly for the
-// warm-up to pay (strongly graded grids), and the y and z passes of k_fit_lines' own range.  Those
+// Lines per block of k_fit_block on an axis of n elements: 32 while two blocks fit an SM, then 16,
+// and 8 while one does (the whole-line sweeps take ten times as long there); 0 where the whole-line
+// sweeps run: longer lines, factors that decay too slowly for the warm-up to pay (strongly graded
+// grids), and the y and z passes of k_fit_lines' own range.  Those
 // passes are coalesced as they are; they lose where there are too few lines to fill the GPU, or
 // where a field is larger than L2 so that their second sweep reads it from HBM again.  Measured on
 // B200 (FP64, three components, us, whole-line sweep against this):
-//   x: 48^3 22.8 / 10.5, 101x75x50 39 / 15, 173x160x147 137 / 81, 256^3 511 / 274, 1001x487x8 456 / 134
+//   x: 48^3 22.8 / 10.5, 101x75x50 39 / 15, 173x160x147 137 / 81, 256^3 511 / 274, 1001x487x8 457 / 100,
+//      1001x487 394 / 36, 1401x487 547 / 52, 1700x487 674 / 56
 //   y: 48^3 14.6 / 10.5, 101x75x50 18.7 / 20.5, 128^3 42 / 46, 200^3 190 / 135, 256^3 342 / 305,
 //      1001x487x8 151 / 93;  z of 8 planes (1001x487x8): 74 / 381
 // Bound by the L1/shared data pipe on large grids (65 to 76 % at 256^3, DRAM 34 %: the staged
 // values of a chunk are read for its neighbours' warm-ups too).
+// Under 32 lines per block a warp sweeps 2 or 4 chunks at once.  With the interior rows' factors in
+// shared memory and chunk lengths that keep those chunks in different banks the x fit of a 1001 x 487
+// plane took 50 -> 36 us (in a run, among other fields: 125 -> 73, and its y fit 88 -> 59).
 constexpr int FITB_MAX_WARM = 96;
 template <typename T>
 inline int fit_block_lines(int n, int warm, int axis, long nlines) {
   if (warm <= 0 || warm > FITB_MAX_WARM) return 0;
   if (axis != 0 && (n < 24 || (nlines > 5000 && 3.0 * n * nlines * sizeof(T) < 128e6))) return 0;
   for (int lines = 32; lines >= 8; lines /= 2)
-    if ((size_t)n * (lines + 1) * sizeof(T) <= 112 * 1024) return lines;
+    if ((size_t)n * (lines + 1 + (lines < 32 ? 3 : 0)) * sizeof(T) <= (size_t)(lines > 8 ? 112 : 168) * 1024) return lines;
   return 0;
 }
 
@@ -1463,7 +1496,7 @@ inline void fit_block_launch(const SplineAxis<T> &A, const FieldPtrs<T> &s, cons
                              long nz, cudaStream_t stream) {
   const long nlines = axis == 0 ? ny * nz : (axis == 1 ? sx * nz : sxy);
   const dim3 grd((unsigned)((nlines + LINES - 1) / LINES), 3);
-  const size_t smem = (size_t)A.n * (axis == 0 ? LINES + 1 : LINES) * sizeof(T);
+  const size_t smem = (size_t)A.n * ((axis == 0 ? LINES + 1 : LINES) + (LINES < 32 ? 3 : 0)) * sizeof(T);
   if (axis == 0) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_fit_block<T, K, true, ADJ, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_fit_block<T, K, true, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, nlines, nlines, sx, 0);
