@@ -85,7 +85,8 @@ void cfd2lcs_get_phase_times_c(double t[7]);
 
 /* Device time of the hot kernels alone (CUDA events around each launch), cumulative:
  * t[0] backward semi-Lagrangian subcycle kernels, t[1] forward particle kernels (ms);
- * n[0], n[1] the number of launches timed. */
+ * n[0], n[1] the number of subcycles they advanced: one per launch, except that small LINEAR sets
+ * advance several in one launch. */
 void cfd2lcs_get_kernel_times_c(double t[2], long long n[2]);
 
 /* Launches of the B-spline subcycle kernels that stage their coefficient taps in shared

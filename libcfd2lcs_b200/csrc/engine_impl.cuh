@@ -785,10 +785,10 @@ class Engine : public EngineBase {
       if (sp.tune >= 0) tune_record(sp.tune, ms);
       if (sp.kind == SPAN_SL) {
         counters_.sl_kernel_ms += ms;
-        counters_.sl_kernel_launches++;
+        counters_.sl_kernel_launches += sp.sub;
       } else if (sp.kind == SPAN_FWD) {
         counters_.fwd_kernel_ms += ms;
-        counters_.fwd_kernel_launches++;
+        counters_.fwd_kernel_launches += sp.sub;
         if (sp.diag >= 0 && sp.diag < (int)diags_.size()) {
           DiagT &d = diags_[sp.diag];
           const double each = (double)ms / sp.sub;  // per subcycle
