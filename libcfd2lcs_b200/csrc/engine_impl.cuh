@@ -647,7 +647,7 @@ class Engine : public EngineBase {
           // more time to disorder than a sort costs (sort_due)
           const int di = (int)(&d - diags_.data());
           const bool resort =
-              usable ? d.since_sort >= sort_interval(d) || (tile_mode_ == 2 && d.fwd_variant != 1) : sort_due(d);
+              usable ? d.since_sort >= sort_interval() || (tile_mode_ == 2 && d.fwd_variant != 1) : sort_due(d);
           if (resort) {
             d.fwd_variant = usable ? tile_variant(1) : 0;
             if (!usable) {
@@ -2334,18 +2334,15 @@ class Engine : public EngineBase {
   // subcycles, so that the particles of a block gather neighbouring spline taps as the SL
   // kernel's blocks do.  Results do not depend on the order: every particle is advanced
   // independently and the snapshot reads it back through the inverse map.  Measured on B200
-  // (ABC 256^3, RK3 CUBIC, FP64): every 6 / 4 / 3 / 2 subcycles gave 332.9 / 330.9 / 328.9 /
-  // 326.0 ms per update (the forward launch 7.55 -> 6.94 ms against 0.9 ms per sort).
+  // (ABC 256^3, RK3 CUBIC, FP64, 0.8 ms a sort), every 1 / 2 / 3 / 4 subcycles: in the first 51
+  // subcycles after a reset, where the node order still helps, 556 / 546 / 543 / 543 ms per pass;
+  // over a horizon of some hundred (dt = 0.05, h = 1) 267.9 / 272.2 / 276.8 / 280.3 ms per update.
 #ifndef CFD2LCS_SORT_INTERVAL
 #define CFD2LCS_SORT_INTERVAL 2
 #endif
   static constexpr int kSortInterval = CFD2LCS_SORT_INTERVAL;
-  // The gathering B-spline kernel in the long rows of gather_tiles: every 1 / 2 / 3 / 4 subcycles
-  // 244.0 / 253.1 / 258.1 / 260.1 ms of launches per pass of 51 at ABC 256^3, and 0.8 ms a sort:
-  // 556 / 546 / 543 / 543 ms per pass in all.
-  static constexpr int kGatherSortInterval = 4;
   int sort_every_ = 0;  // CFD2LCS_B200_SORT_EVERY at cfd2lcs_init (0: the default below)
-  long sort_interval(const DiagT &d) const { return sort_every_ > 0 ? sort_every_ : (d.fwd_variant == 1 ? kSortInterval : kGatherSortInterval); }
+  long sort_interval() const { return sort_every_ > 0 ? sort_every_ : kSortInterval; }
   // Re-sort schedule of a set whose forward kernel gathers (not the staged family): a sort
   // restores the coalescing the launches lose as the particles drift from the order of the
   // last sort, so it pays once the time they have lost since that sort -- each launch's event
