@@ -38,7 +38,11 @@ int cfd2lcs_get_ftle_c(int lcs_handle, lcsdata_t *ftle);
 int cfd2lcs_get_flowmap_c(int lcs_handle, lcsdata_t *fm);
 
 /* cfd2lcs_update_c with u, v, w already resident in device memory (n[0]*n[1]*n[2] values
- * each, i fastest, same precision as lcsdata_t); no host copies. */
+ * each, i fastest, same precision as lcsdata_t); no host copies.
+ * Ordering: an update, this form or cfd2lcs_update_c, starts after the work queued so far on the
+ * default stream of the current device (the legacy default stream, and so on the streams that
+ * synchronise with it).  Work on streams created with cudaStreamNonBlocking is waited for only if
+ * the default stream waits for it.  The update is complete when the call returns. */
 void cfd2lcs_update_device_c(int n[3], const lcsdata_t *d_u, const lcsdata_t *d_v, const lcsdata_t *d_w, lcsdata_t time);
 
 /* Velocity invariants of a diagnostic's latest frame, computed when the option
@@ -149,7 +153,8 @@ int cfd2lcs_batch_add_c(const int n[3], const lcsdata_t *x, const lcsdata_t *y, 
 int cfd2lcs_batch_diagnostic_init_c(int id, int lcs_type, lcsdata_t T, lcsdata_t h);
 
 /* One update of `count` instances: ids[q] receives the device-resident velocity d_u[q],
- * d_v[q], d_w[q] (n[0]*n[1]*n[2] values of that instance, i fastest) at time[q]. */
+ * d_v[q], d_w[q] (n[0]*n[1]*n[2] values of that instance, i fastest) at time[q].  Ordered after the
+ * caller's work as cfd2lcs_update_device_c is. */
 int cfd2lcs_batch_update_device_c(int count, const int *ids, const lcsdata_t *const *d_u, const lcsdata_t *const *d_v,
                                   const lcsdata_t *const *d_w, const lcsdata_t *time);
 

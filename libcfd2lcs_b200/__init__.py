@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 import numpy as np
 
@@ -142,6 +143,18 @@ def load(precision: str = "dp") -> C.CDLL:
     return lib
 
 
+def _join_current_stream():
+    """The calls that take device pointers run after what is queued on the default stream; this puts
+    PyTorch's current stream, where it is another one, in front of that.  (Nothing runs on a stream
+    that is capturing, so there is nothing to wait for.)"""
+    torch = sys.modules.get("torch")
+    if torch is None or not torch.cuda.is_initialized():
+        return
+    s = torch.cuda.current_stream()
+    if s.cuda_stream and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.default_stream().wait_stream(s)
+
+
 class Cfd2lcs:
     """The reference's entry points on one library instance (process-global state, like the
     Fortran module globals).  Arrays are numpy arrays of shape (ni, nj, nk); they are
@@ -179,7 +192,9 @@ class Cfd2lcs:
         self.lib.cfd2lcs_update_c(self._p(n), self._p(u), self._p(v), self._p(w), self.R(time))
 
     def update_device(self, d_u: int, d_v: int, d_w: int, time):
-        """u, v, w already in device memory (raw device pointers, e.g. tensor.data_ptr())."""
+        """u, v, w already in device memory (raw device pointers, e.g. tensor.data_ptr()).  The
+        call runs after the work queued on PyTorch's current stream and on the default stream."""
+        _join_current_stream()
         n = np.ascontiguousarray(self.n, dtype=np.int32)
         self.lib.cfd2lcs_update_device_c(self._p(n), C.c_void_p(d_u), C.c_void_p(d_v), C.c_void_p(d_w), self.R(time))
 
@@ -368,7 +383,9 @@ class Batch:
         return self.lib.cfd2lcs_batch_diagnostic_init_c(int(inst), int(lcs_type), self.R(T), self.R(h))
 
     def update_device(self, ids, d_u, d_v, d_w, times) -> int:
-        """ids: instance ids; d_u/d_v/d_w: device pointers (ints); times: per instance."""
+        """ids: instance ids; d_u/d_v/d_w: device pointers (ints); times: per instance.  Ordered after
+        the caller's work as Cfd2lcs.update_device is."""
+        _join_current_stream()
         k = len(ids)
         I = np.ascontiguousarray(ids, dtype=np.int32)
         U = (C.c_void_p * k)(*d_u)
@@ -409,7 +426,8 @@ def adjoint_ftle(grid, u, v, w, times, weight, integrator=2, cfl=0.5, checkpoint
                  interpolator=1):
     """J = sum(weight * FTLE) of the backward flow map over all levels and, with gradient,
     dJ/du of every level (cfd2lcs_adjoint_ftle_interp_c; interpolator 1 LINEAR or 3 CUBIC).  u, v, w: lists of CUDA tensors, one per
-    level (n[0]*n[1]*n[2] values, i fastest, the library's precision); weight: CUDA tensor.
+    level (n[0]*n[1]*n[2] values, i fastest, the library's precision); weight: CUDA tensor; work still
+    queued on them, on PyTorch's current stream or the default stream, runs first.
     Returns (J, gu, gv, gw) with gu, gv, gw lists of CUDA tensors (None without gradient)."""
     import torch
     lib = load(precision)
@@ -427,6 +445,7 @@ def adjoint_ftle(grid, u, v, w, times, weight, integrator=2, cfl=0.5, checkpoint
     msg = C.create_string_buffer(512)
     p = lambda a: a.ctypes.data_as(C.c_void_p)
     fl = np.asfortranarray(grid.flag, dtype=np.int32).ravel(order="F")
+    _join_current_stream()
     rc = lib.cfd2lcs_adjoint_ftle_interp_c(p(n), p(xs), p(ys), p(zs), p(fl), int(integrator), int(interpolator), R(cfl), L,
                                            C.cast(ptrs(u), C.c_void_p), C.cast(ptrs(v), C.c_void_p), C.cast(ptrs(w), C.c_void_p), p(tm),
                                            C.c_void_p(weight.data_ptr()), int(checkpoint_every), C.byref(J),
@@ -442,7 +461,7 @@ def adjoint_ftle(grid, u, v, w, times, weight, integrator=2, cfl=0.5, checkpoint
 def tangent_ftle(grid, u, v, w, times, weight, du, dv, dw, integrator=2, cfl=0.5, precision="dp", interpolator=1):
     """J and dJ = <dJ/du, d> of the adjoint's objective for one direction d = (du, dv, dw) (lists of
     CUDA tensors, one per level, like u, v, w), by the tangent-linear sweep
-    (cfd2lcs_tangent_ftle_c).  Returns (J, dJ)."""
+    (cfd2lcs_tangent_ftle_c).  Returns (J, dJ).  Ordered after the caller's work as adjoint_ftle is."""
     lib = load(precision)
     dt = np.float64 if precision == "dp" else np.float32
     R = C.c_double if precision == "dp" else C.c_float
@@ -455,6 +474,7 @@ def tangent_ftle(grid, u, v, w, times, weight, du, dv, dw, integrator=2, cfl=0.5
     msg = C.create_string_buffer(512)
     p = lambda a: a.ctypes.data_as(C.c_void_p)
     fl = np.asfortranarray(grid.flag, dtype=np.int32).ravel(order="F")
+    _join_current_stream()
     rc = lib.cfd2lcs_tangent_ftle_interp_c(p(n), p(xs), p(ys), p(zs), p(fl), int(integrator), int(interpolator), R(cfl), L, ptrs(u),
                                            ptrs(v), ptrs(w), p(tm), C.c_void_p(weight.data_ptr()), ptrs(du), ptrs(dv), ptrs(dw),
                                            C.byref(J), C.byref(dJ), msg, 512)

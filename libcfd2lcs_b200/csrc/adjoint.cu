@@ -1525,6 +1525,7 @@ class Adjoint {
       cudaStreamSynchronize(stream_);
       cudaStreamDestroy(stream_);
     }
+    if (caller_) cudaEventDestroy(caller_);
   }
 
   bool run(double *J, std::string &msg) {
@@ -1569,6 +1570,9 @@ class Adjoint {
         return false;
       }
     ACK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    // the levels, weight and direction are read, and the gradients written, after the caller's work
+    ACK(cudaEventCreateWithFlags(&caller_, cudaEventDisableTiming));
+    ACK(wait_for_caller(stream_, caller_));
     if (!pool_.open(stream_, msg)) return false;
     std::vector<int> flag((size_t)n[0] * n[1] * n[2], 0);
     if (pr_.flag) std::memcpy(flag.data(), pr_.flag, flag.size() * sizeof(int));
@@ -2263,6 +2267,7 @@ class Adjoint {
   DevGrid<T> dg_{};
   Pool pool_;
   cudaStream_t stream_ = nullptr;
+  cudaEvent_t caller_ = nullptr;
   DevReduce *red_dev_ = nullptr;  // [0]: the sweeps' error word; [1 + l]: ingest of level l
   long N_ = 0, ntot_ = 0;
   std::vector<T *> U_, Ub_, cp_;

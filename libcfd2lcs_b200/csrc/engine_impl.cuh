@@ -178,6 +178,7 @@ class Engine : public EngineBase {
     if (stream_) cudaStreamSynchronize(stream_);
     arena_.release();
     for (auto &e : ev_) cudaEventDestroy(e);
+    if (caller_) cudaEventDestroy(caller_);
     for (auto &e : evpool_) cudaEventDestroy(e);
     if (red_host_) cudaFreeHost(red_host_);
     if (stream_) cudaStreamDestroy(stream_);
@@ -235,6 +236,7 @@ class Engine : public EngineBase {
       CK(cudaEventCreate(&ev));
       ev_.push_back(ev);
     }
+    CK(cudaEventCreateWithFlags(&caller_, cudaEventDisableTiming));
     CK(cudaMallocHost(&red_host_, sizeof(DevReduce)));
     if (const char *e = std::getenv("CFD2LCS_B200_LINEAR_BLEND_MIN")) lin_blend_min_ = std::atol(e);
     if (const char *e = std::getenv("CFD2LCS_B200_TMA_TENSOR")) tma_tensor_ = std::atoi(e) != 0;
@@ -447,6 +449,8 @@ class Engine : public EngineBase {
       return false;
     }
     const int interp = interpolator();
+    // the velocity arrays, and readers of the buffers this update rewrites (cfd2lcs_ftle_device_ptr_c)
+    CK(wait_for_caller(stream_, caller_));
     // --- K0 ingest --------------------------------------------------------------------
     CK(cudaEventRecord(ev_[8], stream_));
     CK(cudaEventRecord(ev_[0], stream_));
@@ -2415,6 +2419,7 @@ class Engine : public EngineBase {
   DevArena arena_;
   cudaStream_t stream_ = nullptr;
   std::vector<cudaEvent_t> ev_;
+  cudaEvent_t caller_ = nullptr;  // the caller's work before an update (wait_for_caller)
   int n_[3] = {0, 0, 0};
   long N_ = 0, ntot_ = 0;
   TV *u_[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
