@@ -53,8 +53,9 @@ enum { LINEAR_I = 1, CUBIC_I = 3 };
 // Device memory of the adjoint calls.  cudaMalloc and cudaFree take 0.25 and 0.2 ms a buffer, and
 // milliseconds where hundreds of MB are mapped and unmapped: 18 of the 29 ms of a gradient at 80^3
 // (39 buffers, 0.4 GB).  The calls draw from one stream-ordered pool per device instead, which keeps up
-// to 1 GiB from one call to the next (an optimisation calls the gradient again and again); what is
-// above that goes back to the device when a call ends, the rest when the library is reset or finalised
+// to 1 GiB from one call to the next (an optimisation calls the gradient again and again) while half
+// of the device's memory is free; what is above that goes back to the device when a call ends, the
+// rest when the library is reset or finalised, or when one of its allocations fails
 // (adjoint_release_memory).
 constexpr uint64_t POOL_KEEP = 1ull << 30;
 std::mutex g_pool_lock;
@@ -2092,7 +2093,9 @@ class Adjoint {
       maxsub = std::max(maxsub, m);
     }
     std::vector<T *> states;
-    if (!slab(states, (size_t)3 * (maxsub + 1), msg)) return false;
+    if (!slab(states, (size_t)3 * maxsub, msg)) return false;
+    // a segment's last state is the map it ends with, which nothing reads: a forward buffer holds it
+    states.insert(states.end(), fm_[0], fm_[0] + 3);
     for (int s = nseg - 1; s >= 0; s--) {
       const int l0 = s * K + 1, l1 = std::min((s + 1) * K, L - 1);
       // recompute the segment from its checkpoint, keeping the flow map before each subcycle
@@ -2291,8 +2294,13 @@ void adjoint_release_memory() {
 }
 
 bool adjoint_ftle(const AdjointProblem &p, double *J, std::string &msg) {
-  Adjoint<lcsdata_t> a(p);
-  return a.run(J, msg);
+  bool ok;
+  {
+    Adjoint<lcsdata_t> a(p);
+    ok = a.run(J, msg);
+  }
+  if (!ample_memory(0)) adjoint_release_memory();
+  return ok;
 }
 
 }  // namespace cfd2lcs

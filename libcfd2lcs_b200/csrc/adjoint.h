@@ -32,7 +32,8 @@ struct AdjointProblem {
 // linear sweep in the same forward pass.  Returns false with msg on error.
 bool adjoint_ftle(const AdjointProblem &p, double *J, std::string &msg);
 
-// Gives the device memory kept between adjoint calls (at most 1 GiB per device) back.
+// Gives the device memory kept between adjoint calls (at most 1 GiB per device) back; safe beside calls
+// in other threads.
 void adjoint_release_memory();
 
 }  // namespace cfd2lcs

@@ -56,6 +56,13 @@ inline cudaError_t wait_for_caller(cudaStream_t stream, cudaEvent_t ev) {
   return e != cudaSuccess ? e : cudaStreamWaitEvent(stream, ev, 0);
 }
 
+// Whether half of the device's memory stays free beside `bytes` more: the condition for buffers that
+// only save time, so that the library's later ones and the caller's own still fit.
+inline bool ample_memory(size_t bytes) {
+  size_t free = 0, total = 0;
+  return cudaMemGetInfo(&free, &total) == cudaSuccess && free >= bytes + total / 2;
+}
+
 template <typename T>
 struct DevGrid {
   GridParams<T> P;

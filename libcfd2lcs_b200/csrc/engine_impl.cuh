@@ -4,10 +4,12 @@
 
 #include "engine.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <memory>
 #include <map>
@@ -16,6 +18,7 @@
 
 #include <cuda.h>
 
+#include "adjoint.h"
 #include "grid.h"
 #include "kernels.cuh"
 #include "launch.h"
@@ -50,18 +53,32 @@ class DevArena {
     for (void *p : ptrs_) cudaFree(p);
     ptrs_.clear();
   }
+  // called when an allocation fails: gives memory back that only saves time
+  std::function<void()> reclaim;
   // Every buffer gets 256 bytes of slack past its end: the staged-tile kernels copy rows in
   // whole 16-byte units, so the copy of an array's last row may read up to 15 bytes past it.
   template <typename X>
   X *alloc(size_t n, std::string &msg) {
     void *p = nullptr;
     cudaError_t e = cudaMalloc(&p, n * sizeof(X) + 256);
+    if (e == cudaErrorMemoryAllocation && reclaim) {
+      cudaGetLastError();
+      reclaim();
+      e = cudaMalloc(&p, n * sizeof(X) + 256);
+    }
     if (e != cudaSuccess) {
       msg = std::string("device allocation failed: ") + cudaGetErrorString(e);
       return nullptr;
     }
     ptrs_.push_back(p);
     return static_cast<X *>(p);
+  }
+  // before its time (waits for the work that uses it)
+  void free(void *p) {
+    const auto q = std::find(ptrs_.begin(), ptrs_.end(), p);
+    if (q == ptrs_.end()) return;
+    ptrs_.erase(q);
+    cudaFree(p);
   }
 
  private:
@@ -237,6 +254,10 @@ class Engine : public EngineBase {
       ev_.push_back(ev);
     }
     CK(cudaEventCreateWithFlags(&caller_, cudaEventDisableTiming));
+    arena_.reclaim = [this] {
+      release_blends();
+      adjoint_release_memory();
+    };
     CK(cudaMallocHost(&red_host_, sizeof(DevReduce)));
     if (const char *e = std::getenv("CFD2LCS_B200_LINEAR_BLEND_MIN")) lin_blend_min_ = std::atol(e);
     if (const char *e = std::getenv("CFD2LCS_B200_TMA_TENSOR")) tma_tensor_ = std::atoi(e) != 0;
@@ -676,6 +697,7 @@ class Engine : public EngineBase {
       spans_.push_back({adv0, adv1, d.type == FTLE_BKWD ? 1 : 2});
     }
 
+    blends_used_ = false;
     // --- h boundaries: K7 snapshot, K4 composition, K5 FTLE, reset ----------------------
     // (auxiliary sets first: a diagnostic's AUX_GRID FTLE reads their composed maps)
     for (int pass = 0; pass < 2; pass++)
@@ -1143,41 +1165,69 @@ class Engine : public EngineBase {
   // instead of three times, 8 fields moved for 6 blends instead of 12.  The sets of an update share
   // the buffers.  A stage that starts on the node (backward sets on the solver grid) needs no blend.
   // Measured on B200, ABC 256^3, per subcycle: LINEAR RK2 0.237 -> 0.168 ms, CUBIC RK3 0.241 -> 0.155.
+  // The buffers a subcycle cannot do without (its distinct stage fractions, at most 3) are taken when it
+  // first needs them; the others, which only save passes, once an update has several subcycles and
+  // while half of the device's memory stays free, and they are given back when an allocation of
+  // this instance fails (release_blends).
   static constexpr int kBlends = 7;
   TV *blend_[kBlends][3] = {};
   double blend_ct_[kBlends] = {};
   long long blend_update_[kBlends] = {};
-  int nblends_ = 0;
+  int nblends_ = 0, blends_needed_ = 0;
+  bool blends_asked_ = false;  // whether the others were asked for
+  bool blends_used_ = false;   // subcycles that read them are being enqueued
 
-  bool alloc_blends(std::string &msg) {
-    for (int b = 0; b < kBlends; b++) {
-      TV *f[3];
-      for (int c = 0; c < 3; c++)
-        if (!(f[c] = arena_.alloc<TV>(ntot_, msg))) {
-          if (b < 3) return false;
-          cudaGetLastError();  // no room: three buffers serve one subcycle at a time
-          msg.clear();
-          return true;
-        }
-      for (int c = 0; c < 3; c++) blend_[b][c] = f[c];
-      blend_update_[b] = -1;
-      nblends_ = b + 1;
-    }
+  bool add_blend(std::string &msg) {
+    TV *f[3] = {};
+    for (int c = 0; c < 3; c++)
+      if (!(f[c] = arena_.alloc<TV>(ntot_, msg))) {
+        while (c-- > 0) arena_.free(f[c]);
+        return false;
+      }
+    for (int c = 0; c < 3; c++) blend_[nblends_][c] = f[c];
+    blend_update_[nblends_++] = -1;
     return true;
+  }
+
+  bool ensure_blends(int need, bool more, std::string &msg) {
+    blends_needed_ = std::max(blends_needed_, need);
+    while (nblends_ < need)
+      if (!add_blend(msg)) return false;
+    if (!more || blends_asked_) return true;
+    blends_asked_ = true;
+    std::string none;
+    while (nblends_ < kBlends && ample_memory(3 * ntot_ * sizeof(TV)) && add_blend(none)) {
+    }
+    cudaGetLastError();
+    return true;
+  }
+
+  // gives the buffers no subcycle has needed back
+  void release_blends() {
+    while (!blends_used_ && nblends_ > blends_needed_) {
+      nblends_--;
+      for (int c = 0; c < 3; c++) {
+        arena_.free(blend_[nblends_][c]);
+        blend_[nblends_][c] = nullptr;
+      }
+    }
   }
 
   bool stage_blends(const DiagT &d, lcsdata_t t, lcsdata_t dt, long left, VelFields<TV> &V, std::string &msg) {
     static const int nst[5] = {1, 1, 2, 3, 4};
     const int ns = nst[std::min(std::max(opt_->integrator, 0), 4)], s0 = d.type == FTLE_BKWD && !d.lg ? 1 : 0;
     if (s0 == ns) return true;
-    if (!nblends_ && !alloc_blends(msg)) return false;
+    StageTimes S = stage_times(t, dt);
+    int need = 0;  // distinct fractions of this subcycle
+    for (int st = s0; st < ns; st++) need += std::find(S.ct + s0, S.ct + st, S.ct[st]) == S.ct + st;
+    blends_used_ = true;
+    if (!ensure_blends(need, left > 1, msg)) return false;
     const long long upd = counters_.updates;
     auto holder = [&](double ct) {
       for (int b = 0; b < nblends_; b++)
         if (blend_update_[b] == upd && blend_ct_[b] == ct) return b;
       return -1;
     };
-    StageTimes S = stage_times(t, dt);
     bool missing = false;
     for (int st = s0; st < ns; st++) missing = missing || holder(S.ct[st]) < 0;
     if (missing) {
