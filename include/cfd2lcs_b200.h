@@ -180,7 +180,10 @@ void cfd2lcs_batch_reset_c(void);
  * times: host, increasing; d_weight: device, n[0]*n[1]*n[2].  Writes *J and, when d_gu,
  * d_gv, d_gw are not NULL, dJ/du of every level into those device arrays.  Discrete choices
  * of the forward map (subcycle counts, interpolation brackets, clamped weights) are held
- * fixed.  Allocates device memory for the levels, their adjoints and the checkpoints.
+ * fixed.  Allocates device memory for the levels, their adjoints and the checkpoints; up to
+ * 1 GiB of it is kept for the next call if half of the device's memory is free then, until
+ * cfd2lcs_finalize_c, cfd2lcs_reset_c or cfd2lcs_batch_reset_c.
+ * Ordered after the caller's work as cfd2lcs_update_device_c is, and complete on return.
  * Returns 0, or 1 with the reason in msg (at most len bytes). */
 int cfd2lcs_adjoint_ftle_c(const int n[3], const lcsdata_t *x, const lcsdata_t *y, const lcsdata_t *z, int integrator,
                            lcsdata_t cfl, int nlevels, const lcsdata_t *const *d_u, const lcsdata_t *const *d_v,

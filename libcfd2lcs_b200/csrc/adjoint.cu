@@ -53,13 +53,28 @@ enum { LINEAR_I = 1, CUBIC_I = 3 };
 // Device memory of the adjoint calls.  cudaMalloc and cudaFree take 0.25 and 0.2 ms a buffer, and
 // milliseconds where hundreds of MB are mapped and unmapped: 18 of the 29 ms of a gradient at 80^3
 // (39 buffers, 0.4 GB).  The calls draw from one stream-ordered pool per device instead, which keeps up
-// to 1 GiB from one call to the next (an optimisation calls the gradient again and again) while half
-// of the device's memory is free; what is above that goes back to the device when a call ends, the
-// rest when the library is reset or finalised, or when one of its allocations fails
-// (adjoint_release_memory).
+// to 1 GiB from one call to the next (an optimisation calls the gradient again and again) if half of
+// the device's memory is free when a call has made it grow (asking takes 0.07 ms, in some runs of a
+// gradient at 80^3 0.8, so calls that find their memory there do not); what is above that goes back to the device when a call ends, the rest
+// when the library is reset or finalised, or when one of its allocations fails (adjoint_release_memory).
 constexpr uint64_t POOL_KEEP = 1ull << 30;
 std::mutex g_pool_lock;
 cudaMemPool_t g_pools[64] = {};
+uint64_t g_kept[64] = {};  // reserved by the pool after the last call that looked
+
+// after a call, its buffers given back
+void keep_or_release() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> guard(g_pool_lock);
+  uint64_t held = 0;
+  if (!g_pools[dev] || cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) return;
+  if (held > g_kept[dev] && !ample_memory(0)) {
+    cudaMemPoolTrimTo(g_pools[dev], 0);
+    held = 0;
+  }
+  g_kept[dev] = held;
+}
 
 bool call_pool(cudaMemPool_t &pool, std::string &msg) {
   int dev = 0;
@@ -2289,8 +2304,11 @@ class Adjoint {
 
 void adjoint_release_memory() {
   std::lock_guard<std::mutex> guard(g_pool_lock);
-  for (cudaMemPool_t p : g_pools)
-    if (p) cudaMemPoolTrimTo(p, 0);
+  for (int dev = 0; dev < 64; dev++)
+    if (g_pools[dev]) {
+      cudaMemPoolTrimTo(g_pools[dev], 0);
+      g_kept[dev] = 0;
+    }
 }
 
 bool adjoint_ftle(const AdjointProblem &p, double *J, std::string &msg) {
@@ -2299,7 +2317,7 @@ bool adjoint_ftle(const AdjointProblem &p, double *J, std::string &msg) {
     Adjoint<lcsdata_t> a(p);
     ok = a.run(J, msg);
   }
-  if (!ample_memory(0)) adjoint_release_memory();
+  keep_or_release();
   return ok;
 }
 
