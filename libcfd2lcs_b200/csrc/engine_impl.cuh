@@ -674,11 +674,10 @@ class Engine : public EngineBase {
           const bool resort =
               usable ? d.since_sort >= sort_interval() || (tile_mode_ == 2 && d.fwd_variant != 1) : sort_due(d);
           if (resort) {
-            d.fwd_variant = usable ? tile_variant(1) : 0;
             if (!usable) {
               if (!timed_sort(d, msg)) return false;
             } else {
-              if (!sort_particles(d, msg, d.fwd_variant == 1)) return false;
+              if (!sort_particles(d, msg, tile_variant(1) == 1)) return false;
               d.since_sort = 0;
               d.excess_ms = 0;
             }
@@ -2434,8 +2433,9 @@ class Engine : public EngineBase {
     return true;
   }
   // fwd_tile: the 16 x 4 x 4-cell tiles the staged forward kernel reads, else the tiles that suit the
-  // gathering kernel
+  // gathering kernel; the kernel of the launches up to the next sort goes with them
   bool sort_particles(DiagT &d, std::string &msg, bool fwd_tile = false) {
+    d.fwd_variant = fwd_tile ? 1 : 0;
     d.sort_geom = fwd_tile ? sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ) : gather_tiles(n_, opt_->interpolator == QUADRATIC || opt_->interpolator == CUBIC);
     if (!sort_slots(d.P, d.P2, d.pkey, d.pcnt, d.poffs, d.ptsum, (int)dN(d), d.sort_geom, msg)) return false;
     std::swap(d.P, d.P2);
