@@ -1468,14 +1468,25 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
 // Lines per block of k_fit_block on an axis of n elements: 32 while two blocks fit an SM, then 16,
 // and 8 while one does (the whole-line sweeps take ten times as long there); 0 where the whole-line
 // sweeps run: longer lines, factors that decay too slowly for the warm-up to pay (strongly graded
-// grids), and the y and z passes of k_fit_lines' own range.  Those
-// passes are coalesced as they are; they lose where there are too few lines to fill the GPU, or
-// where a field is larger than L2 so that their second sweep reads it from HBM again.  Measured on
-// B200 (FP64, three components, us, whole-line sweep against this):
-//   x: 48^3 22.8 / 10.5, 101x75x50 39 / 15, 173x160x147 137 / 81, 256^3 511 / 274, 1001x487x8 457 / 100,
-//      1001x487 394 / 36, 1401x487 547 / 52, 1700x487 674 / 56
-//   y: 48^3 14.6 / 10.5, 101x75x50 18.7 / 20.5, 128^3 42 / 46, 200^3 190 / 135, 256^3 342 / 305,
-//      1001x487x8 151 / 93;  z of 8 planes (1001x487x8): 74 / 381
+// grids), and the y and z passes of k_fit_lines' own range.  Those passes are coalesced as they
+// are; they lose where there are too few lines to fill the GPU, and on fields somewhat larger than L2,
+// whose second sweep reads them from HBM again.  Measured on B200 (FP64, three components, us,
+// whole-line sweep against this; in brackets lines whose middle third is zero: behind a run of zeros
+// longer than the warm-up a sweep's window is what decays from before the run, so those chunks are
+// swept again, one after the other):
+//   x: 48^3 22.8 / 10.5, 101x75x50 44 / 20 [24], 173x160x147 151 / 90 [135], 200^3 300 / 140 [217],
+//      256^3 531 / 278 [426], 1001x487x8 457 / 100, 1001x487 387 / 38 [86], 1401x487 547 / 52, 1700x487 674 / 56
+//   y: 48^3 14.6 / 10.5, 101x75x50 18.7 / 20.5, 128^3 42 / 46, 176^3 112 / 106 [162], 200^3 201 / 138 [227],
+//      224^3 258 / 192 [312], 256^3 338 / 310 [488], 320^3 644 / 547 [1044], 1001x487 111 / 34 [71],
+//      1001x487x8 151 / 93
+//   z: 176^3 107 / 105 [163], 200^3 190 / 137 [227], 224^3 236 / 192 [317], 256^3 319 / 306 [488],
+//      320^3 610 / 565 [1038], 1001x487x8 (8 planes) 74 / 381
+// So many lines take it in y and z between 180 and 300 MB only, where it is worth most.  Below, the
+// whole-line sweeps are as fast; above, they lose 4 to 15 % and flows with regions at rest would lose
+// more: a CUBIC backward update with the motion inside a ball took 25.8 ms at 256^3 and 46.2 at 300^3
+// with every axis chunked, 23.9 and 40.4 with none, and takes 23.1 and 40.1 with the x axis alone
+// (motion everywhere: 23.4 and 39.3, 25.8 and 43.0, 23.8 and 40.2).  At 200^3 such a flow takes 13.1 ms
+// with every axis and 12.9 with none, motion everywhere 12.3 and 14.0.
 // Bound by the L1/shared data pipe on large grids (65 to 76 % at 256^3, DRAM 34 %: the staged
 // values of a chunk are read for its neighbours' warm-ups too).
 // Under 32 lines per block a warp sweeps 2 or 4 chunks at once.  With the interior rows' factors in
@@ -1485,7 +1496,8 @@ constexpr int FITB_MAX_WARM = 96;
 template <typename T>
 inline int fit_block_lines(int n, int warm, int axis, long nlines) {
   if (warm <= 0 || warm > FITB_MAX_WARM) return 0;
-  if (axis != 0 && (n < 24 || (nlines > 5000 && 3.0 * n * nlines * sizeof(T) < 128e6))) return 0;
+  const double bytes = 3.0 * n * nlines * sizeof(T);
+  if (axis != 0 && (n < 24 || (nlines > 5000 && (bytes < 180e6 || bytes > 300e6)))) return 0;
   for (int lines = 32; lines >= 8; lines /= 2)
     if ((size_t)n * (lines + 1 + (lines < 32 ? 3 : 0)) * sizeof(T) <= (size_t)(lines > 8 ? 112 : 168) * 1024) return lines;
   return 0;
