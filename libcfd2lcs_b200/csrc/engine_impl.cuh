@@ -129,6 +129,7 @@ struct Diag {
   SortTiles sort_geom{};  // cell tiles of the last sort (the staged forward kernel reads one tile per block)
   int fwd_variant = 0;    // forward kernel until the next sort: 0 gathering, 1 staged
   long since_sort = 1L << 40;  // forward subcycles since the particles were last sorted (or reset)
+  long since_reset = 0;        // and since they were on their nodes
   // event-timed cost of the last sort, launch time right after it, and the launch time lost
   // since then (gathering forward kernels: the re-sort schedule of sort_due)
   double sort_ms = 0, base_ms = -1, excess_ms = 0;
@@ -361,7 +362,8 @@ class Engine : public EngineBase {
       if (!(d.P.slot = arena_.alloc<int>(dn, msg))) return false;
       d.P2.slot = d.P.slot;  // the inverse map is rewritten whole by every permutation
       // key space for either tile shape of the sort (gathering or staged forward kernel)
-      const long ncell = std::max({sort_key_space(gather_tiles(n_, false)), sort_key_space(gather_tiles(n_, true)),
+      const long ncell = std::max({sort_key_space(gather_tiles(n_, false, sizeof(TV), 0)), sort_key_space(gather_tiles(n_, true, sizeof(TV), 0)),
+                                   sort_key_space(gather_tiles(n_, true, sizeof(TV), 1L << 30)),
                                    sort_key_space(sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ))});
       if (ncell > (long)std::numeric_limits<int>::max()) {
         msg = "diagnostic_init: grid too large for the forward particle sort";
@@ -421,7 +423,7 @@ class Engine : public EngineBase {
     }
     if (!(cp_[0].slot = arena_.alloc<int>(N_, msg))) return false;
     cp_[1].slot = cp_[0].slot;
-    const long ncell = std::max(sort_key_space(gather_tiles(n_, false)), sort_key_space(gather_tiles(n_, true)));
+    const long ncell = sort_key_space(compose_tiles(n_));
     if (ncell > (long)std::numeric_limits<int>::max()) {
       msg = "diagnostic_init: grid too large for the composition sort";
       return false;
@@ -633,6 +635,7 @@ class Engine : public EngineBase {
         const bool timed = d.type == FTLE_FWD;
         spans_.push_back({k0, k1, kkind, -1, timed ? (int)(&d - diags_.data()) : -1, (int)std::min(d.since_sort, 1L << 30), R.n});
         if (timed) d.since_sort += R.n;
+        d.since_reset += R.n;
         sc += R.n;
       }
       for (long sc = 0; !run && sc < nsub; sc++) {
@@ -689,6 +692,7 @@ class Engine : public EngineBase {
           spans_.push_back({k0, k1, kkind, usable && tune_[1].choice < 0 && tile_mode_ == 1 ? 2 + d.fwd_variant : -1, usable ? -1 : di,
                             (int)std::min(d.since_sort, 1L << 30)});
           d.since_sort++;
+          d.since_reset++;
         }
         lp_time = lp_time + dt;
       }
@@ -2071,7 +2075,7 @@ class Engine : public EngineBase {
   void compose_steps(const SplineAxes<T> &sa, DiagT &d, int m, FieldPtrsW<T> out) {
     const int np = (int)N_, grd = (np + 255) / 256;
     int *err = &red_->err;
-    const SortTiles st = gather_tiles(n_, interp_is_spline(I));
+    const SortTiles st = compose_tiles(n_);
     std::string dummy;
     if (m == 0)  // no sub-map yet: no displacement
       for (int c = 0; c < 3; c++) cudaMemsetAsync(out.f[c], 0, np * sizeof(T), stream_);
@@ -2369,7 +2373,7 @@ class Engine : public EngineBase {
   void launch_reset(DiagT &d) {
     const dim3 blk(32, 8, 1);
     counters_.kernel_launches++;
-    d.since_sort = 0;  // the particles are back on their nodes, in node order
+    d.since_sort = d.since_reset = 0;  // the particles are back on their nodes, in node order
     d.fwd_variant = 0;  // which is not the staged kernel's
     d.base_ms = -1;
     d.excess_ms = 0;
@@ -2436,7 +2440,8 @@ class Engine : public EngineBase {
   // gathering kernel; the kernel of the launches up to the next sort goes with them
   bool sort_particles(DiagT &d, std::string &msg, bool fwd_tile = false) {
     d.fwd_variant = fwd_tile ? 1 : 0;
-    d.sort_geom = fwd_tile ? sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ) : gather_tiles(n_, opt_->interpolator == QUADRATIC || opt_->interpolator == CUBIC);
+    d.sort_geom = fwd_tile ? sort_tiles(n_, FWT_TX, FWT_TY, FWT_TZ) : gather_tiles(n_, opt_->interpolator == QUADRATIC || opt_->interpolator == CUBIC, sizeof(TV),
+                                                                                                  d.since_reset);
     if (!sort_slots(d.P, d.P2, d.pkey, d.pcnt, d.poffs, d.ptsum, (int)dN(d), d.sort_geom, msg)) return false;
     std::swap(d.P, d.P2);
     return true;

@@ -894,7 +894,7 @@ constexpr int SORT_TILE = 2048;  // 256 threads x 8 counts
 // Cell tiles of the order: tx x ty x tz cells (tx ty tz = 256), x fastest inside a tile and
 // tiles in x, y, z order; cells c_a in 0..n_a per axis, padded to whole tiles.  The staged forward
 // kernel takes 16 x 4 x 4 (its shared-memory box is that tile widened by 4 cells), the gathering
-// kernels gather_tiles.
+// one gather_tiles, the composition compose_tiles.
 struct SortTiles {
   int tx, ty, tz;     // cells per tile along each axis
   int ntx, nty, ntz;  // tiles along each axis
@@ -911,18 +911,37 @@ __host__ __device__ inline SortTiles sort_tiles(const int n[3], int tx, int ty, 
   return s;
 }
 
-// The gathering kernels' tiles.  B-splines: rows of up to 128 cells, two deep in y.  About one particle
-// lies in a cell, so a warp spans some 32 cells of the order, and every row it crosses into costs
-// its 64 taps another one or two L1 lines per request: long rows are crossed rarely, and that
-// matters more than the rows a block shares in y and z.  Measured on B200 (ABC 256^3 CUBIC FP64,
-// forward launch, sorted every 2): 32 x 4 x 2 5.24 ms, 64 x 2 x 2 5.08, 64 x 4 x 1 5.04, 128 x 2 x 1
-// 4.96, 256 x 1 x 1 4.91, 16 x 8 x 2 5.53; 101 x 75 x 50: 143 us, 128 x 2 x 1 133.  The 8 taps of
-// the others have the larger share of their lines in y and z: 32 x 4 x 2 (200^3 turbulence in FP32
-// 96.4 ms per pass, 128 x 2 x 1 100.0; ABC 256^3 FP64 even).
-__host__ __device__ inline SortTiles gather_tiles(const int n[3], bool spline) {
-  const int tx = !spline || n[0] < 48 ? 32 : (n[0] < 96 ? 64 : 128);
-  return sort_tiles(n, tx, spline ? 256 / tx : 4, spline ? 1 : 2);
+// The gathering forward kernels' tiles.  About one particle lies in a cell, so a warp spans some 32
+// cells of the order, and every row it crosses into costs a B-spline's 64 taps another one or two
+// L1 lines per request; against that stand the rows a block shares in y and z, which count for more
+// the larger the fields and the longer the particles have drifted.  So B-splines take rows of up to
+// 128 cells, two deep in y, and on large grids with FP64 taps 64 x 2 x 2 once the particles have been
+// under way for 32 subcycles.  Measured on B200 (CUBIC RK3,
+// ABC, sorted every 2, ms per subcycle with its share of the sorts; rows / 64 x 2 x 2 / 32 x 4 x 2), in
+// subcycles 16 to 32 after a reset and 256 to 512 (the launch alone in subcycles 0 to 16 at 256^3: 5.23 /
+// 5.29 / 5.38):
+//   FP64  128^3 0.900 / 0.916 / 0.924 and 0.920 / 0.925 / 0.921, 160^3 1.721 / 1.720 / 1.730 and
+//         1.766 / 1.750 / 1.743, 200^3 3.18 / 3.16 / 3.18 and 3.41 / 3.39 / 3.35,
+//         256^3 6.38 / 6.32 / 6.42 and 7.08 / 6.94 / 6.91 (480 subcycles together 7.03 / 6.86 / 6.87)
+//   FP32  128^3 0.559 / 0.581 / 0.585 and 0.556 / 0.575 / 0.572, 256^3 4.03 / 4.10 / 4.18 and
+//         4.33 / 4.38 / 4.36; FP32 velocity alone 256^3 4.26 / 4.34 / 4.39 and 4.55 / 4.63 / 4.59
+//   planes, FP64: 1001 x 487 0.147 / 0.148 / 0.148, 2048 x 1024 0.510 / 0.485 / 0.482,
+//         4096 x 2048 1.98 / 1.88 / 1.91
+// The 8 taps of the others have the larger share of their lines in y and z: 32 x 4 x 2 (200^3
+// turbulence in FP32 96.4 ms per pass, 128 x 2 x 1 100.0; ABC 256^3 FP64 even).
+// taps: bytes of a tap; since: subcycles since the particles left their nodes.
+__host__ __device__ inline SortTiles gather_tiles(const int n[3], bool spline, size_t taps, long since) {
+  if (!spline) return sort_tiles(n, 32, 4, 2);
+  const bool large = since >= 32 && taps == 8 && (long)n[0] * n[1] * n[2] >= (n[2] < 8 ? 1L << 20 : 1L << 22);
+  const int tx = n[0] < 48 ? 32 : (n[0] < 96 || large ? 64 : 128);
+  return sort_tiles(n, tx, (large ? 128 : 256) / tx, large ? 2 : 1);
 }
+
+// The composition's: 32 x 4 x 2 for every interpolator, its particles being further apart (CUBIC, ms per
+// frame, rows of 128 x 2 x 1 / 64 x 2 x 2 / 32 x 4 x 2: 256^3 FP64 43.6 / 43.0 / 41.7 for 10 sub-maps
+// with h = 1, 13.6 / 13.4 / 13.1 for 4 with h = 1/8; 128^3 5.52 / 5.46 / 5.30; 256^3 FP32
+// 31.9 / 31.4 / 30.2; a 2048 x 1024 plane 2.78 / 2.73 / 2.71).
+__host__ __device__ inline SortTiles compose_tiles(const int n[3]) { return sort_tiles(n, 32, 4, 2); }
 
 __host__ __device__ inline long sort_key_space(const SortTiles &s) { return (long)s.ntz * s.nty * s.ntx * 256; }
 

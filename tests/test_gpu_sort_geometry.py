@@ -54,3 +54,34 @@ def test_a_sort_for_another_kernel_ends_the_staged_one():
     assert n == 0
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [(162, 162, 162), (40, 330, 330), (1030, 1024, 1)])
+def test_large_grid_tiles_keep_bits(n):
+    """The 64 x 2 x 2 (32 x 4 x 2 on short rows) tiles of large FP64 grids against particles that are
+    never sorted: particles are advanced one by one, so the order of their slots changes nothing."""
+    import libcfd2lcs_b200 as L
+    api = L.Cfd2lcs("dp")
+    out = []
+    for every in ("1", "1000000"):
+        env = {"CFD2LCS_B200_SL_TILE": "0", "CFD2LCS_B200_SORT_EVERY": every}
+        os.environ.update(env)
+        try:
+            api.reset()
+            g = W.double_gyre_grid(*n[:2]) if n[2] == 1 else W.abc_grid(n[0], nj=n[1], nk=n[2])
+            api.init(g.n, g.x, g.y, g.z, g.flag)
+        finally:
+            for k in env:
+                os.environ.pop(k, None)
+        dt = (40 if n[2] == 1 else 14) / max(n)  # the second update passes 32 subcycles, where the tiles change
+        h = api.diagnostic_init(SC.FTLE_FWD, 0, 2 * dt, 2 * dt, "f")
+        api.set_option("INTEGRATOR", 2)
+        api.set_option("INTERPOLATOR", 3)
+        vel = W.double_gyre_velocity if n[2] == 1 else W.abc_velocity
+        for k in range(3):
+            api.update(*vel(g, 0.0), k * dt)
+        assert api.error()[0] == 0, api.error()
+        out.append((api.flowmap(h), api.counters()["kernel_launches"]))
+    api.reset()
+    assert out[0][1] > out[1][1]  # it was sorted
+    assert np.array_equal(out[0][0], out[1][0])
