@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
@@ -796,8 +797,9 @@ class Engine : public EngineBase {
       d.have_frame = true;
       if (!d.aux_parent) counters_.ftle_frames++;
     }
-    // the device error word comes back with the update's last event
-    CK(cudaMemcpyAsync(&red_host_->err, &red_->err, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    // the device error word and the fits' count come back with the update's last event
+    static_assert(offsetof(DevReduce, redo) == offsetof(DevReduce, err) + sizeof(int), "read back together");
+    CK(cudaMemcpyAsync(&red_host_->err, &red_->err, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_));
     CK(cudaEventRecord(ev_[9], stream_));
     return true;
   }
@@ -842,6 +844,7 @@ class Engine : public EngineBase {
         return false;
       }
     }
+    watch_fits(red_host_->redo);
     red_err_ |= red_host_->err;
     return red_err_ ? err_msg(msg) : true;
   }
@@ -1370,13 +1373,32 @@ class Engine : public EngineBase {
     return true;
   }
 
+  // Chunked fits whose chunks are swept again cost more than the whole-line sweeps where there are many
+  // lines in y and z, and whether a flow's are hardly changes from one update to the next: once an
+  // update's fits swept more than one chunk per block again, the next 64 updates take the whole-line
+  // sweeps, which give the same bits.  (Random lines have 0.00 per block, constant ones, as the ABC
+  // flow's, 0.25, lines with zeros behind or in front of the motion 4 to 5, where the fit takes 1.1 to
+  // 1.6 times the whole-line sweeps' time at 200^3 to 300^3.)
+  int fit_whole_ = 0;    // updates left with whole-line sweeps
+  long fit_blocks_ = 0;  // blocks of this update's watched fits
+  void watch_fits(unsigned redone) {
+    if (fit_whole_ > 0) fit_whole_--;
+    else if ((long)redone > fit_blocks_) fit_whole_ = 64;
+    fit_blocks_ = 0;
+  }
+
   static std::vector<lcsdata_t> pull_table(const SplineAxisHost<lcsdata_t> &A) { return spline_pull_table(A); }
 
   template <typename D, int K>
   void fit_pass(const SplineAxis<D> &A, FieldPtrs<D> s, FieldPtrsW<D> d, int axis, const DevGrid<T> &g) {
     const int sx = g.P.sx, sxy = g.P.sxy, ny = g.P.n[1] + 2, nz = g.P.n[2] + 2;
     counters_.kernel_launches++;
-    if (fit_block<D, K, false>(A, s, d, axis, sx, sxy, ny, nz, stream_)) return;
+    const long nlines = axis == 1 ? (long)sx * nz : sxy;
+    const bool watched = axis != 0 && nlines > FITB_MANY;
+    if (fit_block<D, K, false>(A, s, d, axis, sx, sxy, ny, nz, stream_, fit_whole_ > 0, watched ? &red_->redo : nullptr)) {
+      if (watched) fit_blocks_ += 3 * ((nlines + 31) / 32);
+      return;
+    }
     if (axis == 0) {
       const long warps = (long)((ny + 31) / 32) * nz;
       const size_t smem = sizeof(D) * 4 * 2 * 32 * (XFIT_W + 1);  // two 32 x (XFIT_W + 1) tiles per warp

@@ -26,7 +26,7 @@ struct DevReduce {
   unsigned long long cmax;  // bits of the largest sum_i |u_i| / delta_i (non-negative double)
   unsigned long long cmin;  // bits of the smallest
   int err;
-  int pad;
+  unsigned redo;  // chunks of the update's y and z fits that were swept again (k_fit_block)
 };
 
 template <typename T>
@@ -1369,11 +1369,11 @@ __device__ __forceinline__ bool same_bits(double a, double b) { return __double_
 __device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_int(a) == __float_as_int(b); }
 
 // XPASS: line L is the contiguous row at L * es.  Else line L starts at L % nfast + (L / nfast) *
-// so and its elements are es apart.
+// so and its elements are es apart.  redo (may be null): counts the chunks that were swept again.
 template <typename T, int K, bool XPASS, bool ADJ, int LINES>
 __global__ void __launch_bounds__(FITB_THREADS, 3)
     k_fit_block(const T *__restrict__ pc, int n, int warm, int m0, int m1, const __grid_constant__ FieldPtrs<T> src,
-                const __grid_constant__ FieldPtrsW<T> dst, long nfast, long nlines, long es, long so) {
+                const __grid_constant__ FieldPtrsW<T> dst, long nfast, long nlines, long es, long so, unsigned *redo) {
   extern __shared__ __align__(16) unsigned char fit_smem[];
   T *const tile = reinterpret_cast<T *>(fit_smem);
   constexpr int P = fitb_pitch<XPASS, LINES>(), NCH = FITB_THREADS / LINES;
@@ -1437,11 +1437,16 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
     return r;
   };
   before(win);
+  // (the threads of a warp that sweep a chunk again count as one)
+  auto count = [&] {
+    if (redo && (threadIdx.x & 31) == (unsigned)__ffs(__activemask()) - 1) atomicAdd(redo, 1u);
+  };
   if (__syncthreads_or(some && c0 > 0 && differs(win, wf))) {
     for (int c = 1; c < NCH; c++) {
       if (ck == c && some) {
         before(win);
         if (differs(win, wf)) {
+          count();
 #pragma unroll
           for (int q = 0; q < 3; q++) wf[q] = win[q];
           fit_sweep<T, K, true, ADJ, SM, true>(C, s + off, ep, col, P, c0, c1, m0, m1, win);
@@ -1464,6 +1469,7 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
       if (ck == c && some) {
         behind(win);
         if (differs(win, wb)) {
+          count();
           // the chunk's forward values again (the source is still whole), then backward
           fit_sweep<T, K, true, ADJ, SM, true>(C, s + off, ep, col, P, c0, c1, m0, m1, wf);
           fit_sweep<T, K, false, ADJ, SM, true>(C, col, P, col, P, c0, c1, m0, m1, win);
@@ -1500,23 +1506,22 @@ __global__ void __launch_bounds__(FITB_THREADS, 3)
 //      1001x487x8 151 / 93
 //   z: 176^3 107 / 105 [163], 200^3 190 / 137 [227], 224^3 236 / 192 [317], 256^3 319 / 306 [488],
 //      320^3 610 / 565 [1038], 1001x487x8 (8 planes) 74 / 381
-// So many lines take it in y and z between 180 and 300 MB only, where it is worth most.  Below, the
-// whole-line sweeps are as fast; above, they lose 4 to 15 % and flows with regions at rest would lose
-// more: a CUBIC backward update with the motion inside a ball took 25.8 ms at 256^3 and 46.2 at 300^3
-// with every axis chunked, 23.9 and 40.4 with none, and takes 23.1 and 40.1 with the x axis alone
-// (motion everywhere: 23.4 and 39.3, 25.8 and 43.0, 23.8 and 40.2).  At 200^3 such a flow takes 13.1 ms
-// with every axis and 12.9 with none, motion everywhere 12.3 and 14.0.
+// So many lines take it in y and z above 128 MB, as long as they are not swept again: `whole`, which the
+// engine sets while its fits were (Engine::watch_fits), keeps the whole-line sweeps there.  A CUBIC
+// backward update with the motion inside a ball takes 17.1 ms at 224^3, 25.8 at 256^3 and 46.2 at 300^3
+// with every axis chunked and 15.8, 23.1 and 40.1 with the x axis alone (motion everywhere: 16.1, 23.4
+// and 39.3 against 16.5, 23.8 and 40.2).
 // Bound by the L1/shared data pipe on large grids (65 to 76 % at 256^3, DRAM 34 %: the staged
 // values of a chunk are read for its neighbours' warm-ups too).
 // Under 32 lines per block a warp sweeps 2 or 4 chunks at once.  With the interior rows' factors in
 // shared memory and chunk lengths that keep those chunks in different banks the x fit of a 1001 x 487
 // plane took 50 -> 36 us (in a run, among other fields: 125 -> 73, and its y fit 88 -> 59).
 constexpr int FITB_MAX_WARM = 96;
+constexpr long FITB_MANY = 5000;  // lines that fill the GPU one by one
 template <typename T>
-inline int fit_block_lines(int n, int warm, int axis, long nlines) {
+inline int fit_block_lines(int n, int warm, int axis, long nlines, bool whole) {
   if (warm <= 0 || warm > FITB_MAX_WARM) return 0;
-  const double bytes = 3.0 * n * nlines * sizeof(T);
-  if (axis != 0 && (n < 24 || (nlines > 5000 && (bytes < 180e6 || bytes > 300e6)))) return 0;
+  if (axis != 0 && (n < 24 || (nlines > FITB_MANY && (whole || 3.0 * n * nlines * sizeof(T) < 128e6)))) return 0;
   for (int lines = 32; lines >= 8; lines /= 2)
     if ((size_t)n * (lines + 1 + (lines < 32 ? 3 : 0)) * sizeof(T) <= (size_t)(lines > 8 ? 112 : 168) * 1024) return lines;
   return 0;
@@ -1524,17 +1529,17 @@ inline int fit_block_lines(int n, int warm, int axis, long nlines) {
 
 template <typename T, int K, bool ADJ, int LINES>
 inline void fit_block_launch(const SplineAxis<T> &A, const FieldPtrs<T> &s, const FieldPtrsW<T> &d, int axis, long sx, long sxy, long ny,
-                             long nz, cudaStream_t stream) {
+                             long nz, cudaStream_t stream, unsigned *redo = nullptr) {
   const long nlines = axis == 0 ? ny * nz : (axis == 1 ? sx * nz : sxy);
   const dim3 grd((unsigned)((nlines + LINES - 1) / LINES), 3);
   const size_t smem = (size_t)A.n * ((axis == 0 ? LINES + 1 : LINES) + (LINES < 32 ? 3 : 0)) * sizeof(T);
   if (axis == 0) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_fit_block<T, K, true, ADJ, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fit_block<T, K, true, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, nlines, nlines, sx, 0);
+    k_fit_block<T, K, true, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, nlines, nlines, sx, 0, redo);
   } else {
     const long es = axis == 1 ? sx : sxy;
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_fit_block<T, K, false, ADJ, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fit_block<T, K, false, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, es, nlines, es, sxy);
+    k_fit_block<T, K, false, ADJ, LINES><<<grd, FITB_THREADS, smem, stream>>>(A.pull, A.n, A.warm, A.mid0, A.mid1, s, d, es, nlines, es, sxy, redo);
   }
 }
 
@@ -1542,11 +1547,11 @@ inline void fit_block_launch(const SplineAxis<T> &A, const FieldPtrs<T> &s, cons
 // k_fit_block does not apply
 template <typename T, int K, bool ADJ>
 inline bool fit_block(const SplineAxis<T> &A, const FieldPtrs<T> &s, const FieldPtrsW<T> &d, int axis, long sx, long sxy, long ny, long nz,
-                      cudaStream_t stream) {
-  switch (fit_block_lines<T>(A.n, A.warm, axis, axis == 0 ? ny * nz : (axis == 1 ? sx * nz : sxy))) {
-    case 32: fit_block_launch<T, K, ADJ, 32>(A, s, d, axis, sx, sxy, ny, nz, stream); return true;
-    case 16: fit_block_launch<T, K, ADJ, 16>(A, s, d, axis, sx, sxy, ny, nz, stream); return true;
-    case 8: fit_block_launch<T, K, ADJ, 8>(A, s, d, axis, sx, sxy, ny, nz, stream); return true;
+                      cudaStream_t stream, bool whole = false, unsigned *redo = nullptr) {
+  switch (fit_block_lines<T>(A.n, A.warm, axis, axis == 0 ? ny * nz : (axis == 1 ? sx * nz : sxy), whole)) {
+    case 32: fit_block_launch<T, K, ADJ, 32>(A, s, d, axis, sx, sxy, ny, nz, stream, redo); return true;
+    case 16: fit_block_launch<T, K, ADJ, 16>(A, s, d, axis, sx, sxy, ny, nz, stream, redo); return true;
+    case 8: fit_block_launch<T, K, ADJ, 8>(A, s, d, axis, sx, sxy, ny, nz, stream, redo); return true;
   }
   return false;
 }

@@ -2,6 +2,7 @@
 // bit: one line per combination, "<bad values> <name>".  A NaN counts as equal to a NaN.
 #include <cmath>
 #include <cstdio>
+#include <initializer_list>
 #include <random>
 #include <vector>
 
@@ -20,7 +21,7 @@ double value(int field, std::mt19937_64 &g, long l, int e, int n) {
   std::uniform_real_distribution<double> U(-1.0, 1.0);
   const double r = U(g);
   switch (field) {
-    case 1: return 0.3 + 0.001 * (double)(l % 97);  // the same along the line
+    case 1: return 1.7 * std::sin(0.37 * (double)l);  // the same along the line
     case 2: return e < n / 4 ? r : 0.0;
     case 3: return e < n / 3 || e > 2 * n / 3 ? r : 0.0;
     case 4: return r * std::exp2(40.0 * std::sin(0.7 * e));
@@ -156,24 +157,40 @@ void compare(int nx, int ny, int nz, int axis, bool stretched) {
 int main() {
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) return 2;
-  // the rule: lines in y and z with many lines from 180 to 300 MB, x lines up to what a block holds
-  auto rule = [](int n, int warm, int axis, long nlines, int lines) {
-    std::printf("%d rule %s n %d warm %d axis %d: %d lines\n", fit_block_lines<REAL>(n, warm, axis, nlines) != lines, type_name(REAL()), n, warm, axis, lines);
+  // the rule: many lines in y and z above 128 MB and not `whole`, x lines up to what a block holds
+  auto rule = [](int n, int warm, int axis, long nlines, bool whole, int lines) {
+    std::printf("%d rule %s n %d warm %d axis %d whole %d: %d lines\n", fit_block_lines<REAL>(n, warm, axis, nlines, whole) != lines,
+                type_name(REAL()), n, warm, axis, whole, lines);
   };
   const bool dp = sizeof(REAL) == 8;
   for (int axis = 1; axis < 3; axis++) {
-    rule(130, 41, axis, 130 * 130, 0);
-    rule(202, 41, axis, 202 * 202, dp ? 32 : 0);
-    rule(258, 41, axis, 258 * 258, dp ? 0 : 32);
-    rule(302, 41, axis, 302 * 302, 0);
-    rule(23, 41, axis, 100, 0);
-    rule(24, 41, axis, 100, 32);
+    rule(130, 41, axis, 130 * 130, false, 0);
+    rule(202, 41, axis, 202 * 202, false, dp ? 32 : 0);
+    rule(258, 41, axis, 258 * 258, false, 32);
+    rule(258, 41, axis, 258 * 258, true, 0);
+    rule(23, 41, axis, 100, false, 0);
+    rule(24, 41, axis, 100, true, 32);
   }
-  rule(302, 41, 0, 302 * 302, 32);
-  rule(302, FITB_MAX_WARM + 1, 0, 100, 0);
-  rule(1792, 41, 0, 100, 8);
-  if (dp) rule(1793, 41, 0, 100, 0);
-  else rule(3584, 41, 0, 100, 8), rule(3585, 41, 0, 100, 0);
+  rule(302, 41, 0, 302 * 302, true, 32);
+  rule(302, FITB_MAX_WARM + 1, 0, 100, false, 0);
+  rule(1792, 41, 0, 100, false, 8);
+  if (dp) rule(1793, 41, 0, 100, false, 0);
+  else rule(3584, 41, 0, 100, false, 8), rule(3585, 41, 0, 100, false, 0);
+  // the count of chunks swept again: below one per block on random lines (and, in FP64, constant ones), above
+  // on lines at rest but for their middle, so that the whole-line sweeps take over there
+  for (const int field : std::initializer_list<int>{0, 1, 6}) {
+    if (field == 1 && !dp) continue;
+    Case<REAL> c(150, 150, 5, 1, 4, false);
+    unsigned *redo, n = 0;
+    cudaMalloc(&redo, sizeof(unsigned));
+    cudaMemset(redo, 0, sizeof(unsigned));
+    c.fill(field);
+    fit_block_launch<REAL, 4, false, 32>(c.A, c.in(c.src), c.out(c.b), 1, 150, 150 * 150, 150, 5, 0, redo);
+    cudaMemcpy(&n, redo, sizeof(unsigned), cudaMemcpyDeviceToHost);
+    cudaFree(redo);
+    const unsigned blocks = 3 * ((150 * 5 + 31) / 32);
+    std::printf("%d count %s %s: %u chunks, %u blocks\n", field == 6 ? n <= blocks : n > blocks, type_name(REAL()), FIELD[field], n, blocks);
+  }
   compare<REAL, 4, 32>(5, 3, 3, 0, false);     // fewer points than chunks
   compare<REAL, 4, 32>(203, 35, 5, 0, false);  // a partial block of lines
   compare<REAL, 4, 32>(203, 35, 5, 0, true);
