@@ -148,11 +148,11 @@ def _join_current_stream():
     PyTorch's current stream, where it is another one, in front of that.  (Nothing runs on a stream
     that is capturing, so there is nothing to wait for.)"""
     torch = sys.modules.get("torch")
-    if torch is None or not torch.cuda.is_initialized():
+    # (the raw handle first: a Stream object per call takes longer than the rest of the call's Python)
+    if torch is None or not torch.cuda.is_initialized() or not torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()):
         return
-    s = torch.cuda.current_stream()
-    if s.cuda_stream and not torch.cuda.is_current_stream_capturing():
-        torch.cuda.default_stream().wait_stream(s)
+    if not torch.cuda.is_current_stream_capturing():
+        torch.cuda.default_stream().wait_stream(torch.cuda.current_stream())
 
 
 class Cfd2lcs:

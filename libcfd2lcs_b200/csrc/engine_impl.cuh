@@ -2122,6 +2122,8 @@ class Engine : public EngineBase {
       for (int c = 0; c < 3; c++) out.f[c] = d.composed[c];
       counters_.slots_composed += m;
       const bool F = dg_.P.has_flags != 0;
+      // (a cubic plane takes the general orders here: the fixed ones, INTERP_SPLINE442, are instantiated
+      // for the node-ordered kernel alone, where most planes are; the bits are the same)
 #define COMPOSE_STEPS(I) (F ? compose_steps<I, true>(sa, d, m, out) : compose_steps<I, false>(sa, d, m, out))
       if (iv == INTERP_NEAREST) COMPOSE_STEPS(INTERP_NEAREST);
       else if (iv == INTERP_LINEAR) COMPOSE_STEPS(INTERP_LINEAR);
