@@ -99,7 +99,7 @@ void cfd2lcs_get_kernel_times_c(double t[2], long long n[2]);
 void cfd2lcs_get_staged_launches_c(long long n[2]);
 
 /* Of the staged backward launches, those of the LINEAR kernel that marches planes of the
- * fields along z (FP64 grids whose rows are a multiple of 16 bytes), cumulative. */
+ * fields along z, cumulative. */
 void cfd2lcs_get_march_launches_c(long long *n);
 
 /* The library times both forms of the cubic / LINEAR subcycle kernels -- taps staged in shared
